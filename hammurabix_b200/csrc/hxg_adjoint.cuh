@@ -20,7 +20,7 @@
 //   x = -e_phi.B
 #pragma once
 
-#include "hxg_integrate.cuh"
+#include "hxg_fp64.cuh"
 
 namespace hxg {
 
@@ -86,12 +86,14 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
   const long long gw =
       ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int C = P.chunks;
-  const int seg = lane >> P.log2_chunks;
-  const int c = lane & (C - 1);
+  // the forward's lanes (fp64_tile): chunks of a pixel S lanes apart
+  const int S = 32 >> P.log2_chunks;
+  const int seg = lane & (S - 1);
+  const int c = lane >> (5 - P.log2_chunks);
   const Hpx h = hpx_make((uint64_t)P.nside);
   // shard `shard` of `nshards` of the shell (the forward's pixels)
   const unsigned long long nest =
-      shard_nest(P, (unsigned long long)gw * (32 >> P.log2_chunks) + seg);
+      shard_nest(P, (unsigned long long)gw * S + seg);
   const bool valid = nest < h.npix;
   uint64_t ring = 0;
   bool live = false;
@@ -111,10 +113,10 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
   // exclusive Faraday-depth prefix F_c of the chunks before this one
   double incl = fdc;
   for (int o = 1; o < C; o <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, incl, o);
+    const double v = __shfl_up_sync(0xffffffffu, incl, o * S);
     if (c >= o) incl += v;
   }
-  double Fc = __shfl_up_sync(0xffffffffu, incl, 1);
+  double Fc = __shfl_up_sync(0xffffffffu, incl, S);
   if (c == 0) Fc = 0.;
   // chunk Q, U in the pixel's (global) phase frame
   double qg = qc, ug = uc;
@@ -126,14 +128,14 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
   }
   double qi = qg, ui = ug;
   for (int o = 1; o < C; o <<= 1) {
-    const double vq = __shfl_up_sync(0xffffffffu, qi, o);
-    const double vu = __shfl_up_sync(0xffffffffu, ui, o);
+    const double vq = __shfl_up_sync(0xffffffffu, qi, o * S);
+    const double vu = __shfl_up_sync(0xffffffffu, ui, o * S);
     if (c >= o) {
       qi += vq;
       ui += vu;
     }
   }
-  const int last = (seg << P.log2_chunks) + C - 1;
+  const int last = (C - 1) * S + seg;
   const double Qp = __shfl_sync(0xffffffffu, qi, last);
   const double Up = __shfl_sync(0xffffffffu, ui, last);
   double Qrun = qi - qg, Urun = ui - ug;  // Q, U of the chunks before this one
@@ -178,20 +180,15 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     long long acc_key = -1;
     double gt = P.em_gt, gpp = P.em_gp, last_index = nan("");
     double fdl = 0.;  // running FD of this chunk
-    long long wlo, whi, slo_unused, shi_unused;
-    ray_window(P, ux, uy, uz, wlo, whi, slo_unused, shi_unused);
-    const long long i0 = max((P.step * c) >> P.log2_chunks, wlo);
-    const long long i1 = min((P.step * (c + 1)) >> P.log2_chunks, whi);
-    for (long long i = i0; i < i1; ++i) {
+    const double u3[3] = {ux, uy, uz};
+    int i0, i1;
+    chunk_range64(P, u3, c, i0, i1);
+    for (int i = i0; i < i1; ++i) {
       const double d = P.d_start + ((double)i + 0.5) * P.delta;
       const double px = ux * d + P.obs[0];
       const double py = uy * d + P.obs[1];
       const double pz = uz * d + P.obs[2];
-      // every sample is tested (the certain window measured slower here)
-      const double len = sqrt(px * px + py * py + pz * pz);
-      if (len < P.gc_r_min || len > P.gc_r_max || pz < P.gc_z_min ||
-          pz > P.gc_z_max)
-        continue;
+      if (!kFast && P.gc_r_min > 0. && sqrt(px * px + py * py + pz * pz) < P.gc_r_min) continue;
       const double p3[3] = {px, py, pz};
       V3<double> Breg{0., 0., 0.};
       double tereg = 0.;

@@ -679,7 +679,7 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
   // CRE grid: the emissivity is integrated per sample (cre_grid_j); the
   // FP32C form scales it by 2^128 into FP32 range and k_t = k_p undo that
   if (P.do_sync && m.cre == HXG_CRE_GRID) {
-    P.k_t = P.k_p = delta * P.i2bt * 0x1p-128;
+    P.k_t = P.k_p = delta * P.i2bt * (fp32 ? 0x1p-128 : 1.);
   }
   // analytic synchrotron emissivity constants (integrator.cc:332-346, 401-415)
   if (P.do_sync && m.cre != HXG_CRE_GRID) {
@@ -696,9 +696,9 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     P.em_3qe = 3. * qe;
     P.em_den_p = 16. * cgs::pi * mec2;
     P.em_const = P.models.cre_const_index;
-    const double a_s = P.em_anum / (P.em_3qe * cgs::fp32_bunit);
+    const double a_s = P.em_anum / (P.em_3qe * (fp32 ? cgs::fp32_bunit : 1.));
     P.a_s = a_s;
-    const double kbase = P.em_n0u * 1.73205081 * P.em_qe3 * cgs::fp32_bunit;
+    const double kbase = P.em_n0u * 1.73205081 * P.em_qe3 * (fp32 ? cgs::fp32_bunit : 1.);
     if (P.em_const) {
       const double idx =
           m.cre == HXG_CRE_ANA ? -m.cre_ana.alpha : -(m.cre_unif.alpha);
@@ -709,7 +709,9 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
       const double e = 0.5 * (idx + 1);
       P.em_pow_kind = (e == -1.) ? 1 : (e == 0. ? 2 : 0);
       P.em_pe = 1. - e;
-      const double ae = std::pow(a_s, e);
+      double ae = std::pow(a_s, e);
+      // bperp_pow64 takes |B_perp|^2 in 2^-40 G^2
+      if (!fp32 && P.em_pe != 2.) ae *= std::pow(2., -20. * P.em_pe);
       P.k_t = kbase / P.em_den_t * ae * P.em_gt * delta * P.i2bt;
       P.k_p = kbase / P.em_den_p * ae * P.em_gp * delta * P.i2bt;
     } else {
@@ -717,18 +719,24 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
       P.k_p = kbase / P.em_den_p * delta * P.i2bt;
     }
   }
+  const DevModels &D = P.models;
+  FastModels &F = P.fast;
+  F.sp_b0 = D.sp_b0;
+  F.sp_irs = 1. / D.sp_rs;
+  F.sp_crs = D.sp_rsun / D.sp_rs;
+  F.sp_ihs = 1. / D.sp_hs;
+  F.sp_sin = D.sp_sin;
+  F.sp_cos = D.sp_cos;
+  F.sp_rsun = D.sp_rsun;
+  F.ex_n0 = D.tex_n0;
+  F.ex_irn = 1. / D.tex_rs;
+  F.ex_ihn = 1. / D.tex_hs;
+  F.rc2_hi = 400. * D.kpc * D.kpc;
+  F.rc2_lo = 9. * D.kpc * D.kpc;
   if (fp32) {
     P.fd_fore = fdfore * delta * cgs::fp32_bunit;
     P.k_dm = delta;
     P.phase_k = 2. * P.lambda2 * P.fd_fore;
-    const DevModels &D = P.models;
-    FastModels &F = P.fast;
-    F.sp_b0 = D.sp_b0;
-    F.sp_irs = 1. / D.sp_rs;
-    F.sp_crs = D.sp_rsun / D.sp_rs;
-    F.sp_ihs = 1. / D.sp_hs;
-    F.sp_sin = D.sp_sin;
-    F.sp_cos = D.sp_cos;
     const double sgn = D.sp_b0 < 0. ? -1. : 1.;
     F.sp_crs_l = F.sp_crs + (D.sp_b0 != 0. ? std::log(std::fabs(D.sp_b0)) : 0.);
     F.sp_sin_s = sgn * D.sp_sin;
@@ -736,13 +744,8 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     F.sp_sinf_s = float(F.sp_sin_s);
     F.sp_cosf_s = float(F.sp_cos_s);
     F.ex_ln0 = D.tex_n0 > 0. ? std::log(D.tex_n0) : 0.;
-    F.ex_n0 = D.tex_n0;
-    F.ex_irn = 1. / D.tex_rs;
-    F.ex_ihn = 1. / D.tex_hs;
     F.r2min = P.gc_r_min * P.gc_r_min;
     F.r2max = P.gc_r_max * P.gc_r_max;
-    F.rc2_hi = 400. * D.kpc * D.kpc;
-    F.rc2_lo = 9. * D.kpc * D.kpc;
     F.sp_sinf = float(D.sp_sin);
     F.sp_cosf = float(D.sp_cos);
     F.cre_ir0 = float(1. / D.cre_r0);
@@ -754,6 +757,23 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     F.pe = float(P.em_pe);
   } else {
     P.fd_fore = fdfore;
+    P.phase_k = 2. * P.lambda2 * fdfore * delta;
+    // in extended precision: one rounding each
+    const long double quarter = 4.L * P.lambda2 / 3.14159265358979323846264338327950288L;
+    P.quarter_i = (double)quarter;
+    P.quarter_k = (double)(quarter * fdfore * delta);
+    F.sp_sin_s = D.sp_b0 * D.sp_sin;
+    F.sp_cos_s = D.sp_b0 * D.sp_cos;
+    F.cre64_R0 = D.cre_R0;
+    F.cre64_ir0 = 1. / D.cre_r0;
+    F.cre64_2iz0 = 2. / std::fabs(D.cre_z0);
+    // largest exponents inside the cuts: r, |z| <= gc_r_max
+    const double rm = P.gc_r_max + D.sp_rsun;
+    const auto below = [](double a) { return std::fabs(a) < 680.; };
+    P.exp_ok = (D.breg != kBregSpiral || below(rm * (std::fabs(F.sp_irs) + std::fabs(F.sp_ihs)))) &&
+               (D.tereg != kTeregExpdisk ||
+                below(rm * (std::fabs(F.ex_irn) + std::fabs(F.ex_ihn)))) &&
+               (D.cre != kCreAna || below(rm * (std::fabs(F.cre64_ir0) + F.cre64_2iz0)));
   }
   // grid groups
   P.ngroups = (int)h->groups.size();
@@ -1714,6 +1734,8 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
     const ShellLaunch &L = f == 0 ? P : Pf;
     Fq.lambda2[f] = L.lambda2;
     Fq.phase_k[f] = L.phase_k;
+    Fq.quarter_k[f] = L.quarter_k;
+    Fq.quarter_i[f] = L.quarter_i;
     Fq.k_t[f] = L.k_t;
     Fq.k_p[f] = L.k_p;
     Fq.tc_a[f] = L.tc_a;
@@ -2945,7 +2967,7 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
     uint64_t step;
     if ((st = build_launch(h, E.models, E.obs, 0, L, step)) != HXG_OK) return bail(st);
     L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) : nullptr;
-    b->fast = b->fast && hxg::fast_models(L);
+    b->fast = b->fast && hxg::fast_models(L) && (b->fp32 || L.exp_ok);
   }
   int per_sm = 0;
   cudaError_t ce = hxg::batch_level_occupancy(b->fp32, b->ngroups, b->ext_any, b->fast, &per_sm);

@@ -8,6 +8,7 @@
 #pragma once
 
 #include "hxg_fp32c.cuh"
+#include "hxg_fp64.cuh"
 #include "hxg_integrate.cuh"
 #include "hxg_internal.h"
 
@@ -114,7 +115,7 @@ __device__ __forceinline__ void batch_level_body(const BatchLevel &B) {
       if (kFp32)
         fp32c_tile<NG, kExt, kFast>(P, gw, lane);
       else
-        fp64_tile<NG, false, kExt, kFast>(P, gw, lane);
+        fp64_tile<NG, kExt, kFast>(P, gw, lane);
     }
   }
 }

@@ -107,26 +107,6 @@ __device__ __forceinline__ void trilinear_f32(const float4 *rec, int ny,
   out[3] = rb.y;
 }
 
-// 2^(j/64) for j = 0..63, correctly rounded to FP64.
-__device__ const double kExp2Tab64[64] = {
-    1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
-    1.0442737824274138, 1.0556451783605572, 1.0671404006768237, 1.0787607977571199,
-    1.0905077326652577, 1.102382583307841, 1.1143867425958924, 1.1265216186082418,
-    1.1387886347566916, 1.1511892299529827, 1.1637248587775775, 1.1763969916502812,
-    1.189207115002721, 1.202156731452703, 1.215247359980469, 1.22848053610687,
-    1.241857812073484, 1.255380757024691, 1.2690509571917332, 1.2828700160787783,
-    1.2968395546510096, 1.3109612115247644, 1.3252366431597413, 1.339667524053303,
-    1.3542555469368927, 1.3690024229745905, 1.383909881963832, 1.3989796725383112,
-    1.4142135623730951, 1.42961333839197, 1.4451808069770467, 1.460917794180647,
-    1.4768261459394993, 1.4929077282912648, 1.5091644275934228, 1.5255981507445384,
-    1.5422108254079407, 1.559004400237837, 1.5759808451078865, 1.593142151342267,
-    1.6104903319492543, 1.6280274218573478, 1.645755478153965, 1.6636765803267364,
-    1.681792830507429, 1.7001063537185235, 1.718619298122478, 1.7373338352737062,
-    1.7562521603732995, 1.7753764925265212, 1.7947090750031072, 1.8142521755003989,
-    1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
-    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951,
-};
-
 // e^a for a < 700 (a below -700 is taken as -700) by table-driven range
 // reduction (Tang, ACM TOMS 15, 1989): k = nearest integer of 64 a / ln2,
 // r = a - k ln2/64 with |r| <= ln2/128, e^a = 2^(k >> 6) 2^((k & 63)/64) e^r,
@@ -216,31 +196,6 @@ struct FixAxis {
   __device__ __forceinline__ void next() { a += s; }
 };
 
-// Sample range [ga, gb) of [i0, i1) in which the ray can be inside the grid
-// box 0 < g < n - 1 on every axis (from the slab intersections in FP64,
-// widened by two samples; the fixed-point test decides each sample).
-__device__ __forceinline__ void grid_window(const ShellLaunch &P, const DevGridGroup &G,
-                                            const double g0[3], const double gv[3],
-                                            int i0, int i1, int &ga, int &gb) {
-  double da = -1e300, db = 1e300;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (gv[k] != 0.) {
-      const double t0 = -g0[k] / gv[k], t1 = (G.gmax[k] - g0[k]) / gv[k];
-      da = fmax(da, fmin(t0, t1));
-      db = fmin(db, fmax(t0, t1));
-    } else if (!(g0[k] > 0. && g0[k] < G.gmax[k])) {
-      db = -1e300;
-    }
-  }
-  ga = i1;
-  gb = i1;
-  if (!(da <= db)) return;
-  const double xa = (da - P.d_start) / P.delta - 0.5, xb = (db - P.d_start) / P.delta - 0.5;
-  ga = (int)fmin(fmax(floor(xa) - 2., (double)i0), (double)i1);
-  gb = (int)fmin(fmax(ceil(xb) + 3., (double)ga), (double)i1);
-}
-
 // 2^x in FP32 (the approximate hardware exponential, as __expf uses it).
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -255,43 +210,6 @@ __device__ __forceinline__ float cre_ana_prof32(const FastModels &F, float rf, f
   const float t = ex2_approx(-fabsf(zf) * F.cre_2iz0_l2);
   const float den = 1.f + t;
   return __fdividef(ex2_approx(fmaf(-rf, F.cre_ir0_l2, F.cre_R0_l2)) * t, den * den);
-}
-
-template <int NF>
-__device__ __forceinline__ void combine_chunks_nf(const ShellLaunch &P, const FreqSet<NF> &Fq,
-                                                  int c, double &dm, double &fd, double si[NF],
-                                                  double sq[NF], double su[NF]) {
-  const int C = P.chunks;
-  if (C == 1) return;
-  // inclusive scan of fd within the segment
-  double incl = fd;
-  for (int o = 1; o < C; o <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (c >= o) incl += v;
-  }
-  double excl = __shfl_up_sync(0xffffffffu, incl, 1);
-  if (c == 0) excl = 0.;
-#pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    if (P.do_sync && c > 0) {
-      double sr, cr;
-      sincos(2. * Fq.lambda2[f] * excl, &sr, &cr);
-      const double q = sq[f] * cr - su[f] * sr;
-      const double u = sq[f] * sr + su[f] * cr;
-      sq[f] = q;
-      su[f] = u;
-    }
-  }
-  for (int o = C >> 1; o > 0; o >>= 1) {
-    dm += shfl_xor_d(dm, o);
-    fd += shfl_xor_d(fd, o);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      si[f] += shfl_xor_d(si[f], o);
-      sq[f] += shfl_xor_d(sq[f], o);
-      su[f] += shfl_xor_d(su[f], o);
-    }
-  }
 }
 
 // Warp gw of shell launch P (32/C pixels, C lanes each) for the NF
@@ -662,17 +580,7 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
 template <int NG, bool kExt, bool kFast = false>
 __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, long long gw, int lane) {
   FreqSet<1> Fq;
-  Fq.lambda2[0] = P.lambda2;
-  Fq.phase_k[0] = P.phase_k;
-  Fq.k_t[0] = P.k_t;
-  Fq.k_p[0] = P.k_p;
-  Fq.tc_a[0] = P.tc_a;
-  Fq.tc_b[0] = P.tc_b;
-  Fq.a_s[0] = P.a_s;
-  Fq.inner[0] = 1;
-  Fq.out[0][0] = P.out[2];
-  Fq.out[0][1] = P.out[3];
-  Fq.out[0][2] = P.out[4];
+  freq_of_launch(P, Fq);
   fp32c_tile<NG, kExt, 1, kFast>(P, Fq, gw, lane);
 }
 

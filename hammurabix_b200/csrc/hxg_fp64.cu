@@ -1,0 +1,29 @@
+// hxg_fp64.cu -- instantiations of the FP64 shell kernels.
+#include "hxg_dispatch.cuh"
+#include "hxg_fp64.cuh"
+#include "hxg_internal.h"
+
+namespace hxg {
+
+// The one-grid kernels read 32-byte records in one load.  Records that the
+// caller packed (hxg_write_grid_noalloc) need be aligned to 16 bytes only;
+// those take the kernel for several grids, whose loads are 16 bytes wide.
+static int shape64(const ShellLaunch &P) {
+  const bool wide = P.ngroups != 1 || (reinterpret_cast<uintptr_t>(P.groups[0].rec) & 31) == 0;
+  return wide ? P.ngroups : kMaxGroups;
+}
+
+cudaError_t launch_shell64(cudaStream_t s, const ShellLaunch &P, unsigned blocks,
+                           unsigned threads) {
+  const bool fast = fast_models(P) && P.exp_ok;
+  return by_shape(shape64(P), P.ext != nullptr, [&](auto ng, auto ext) {
+    constexpr int NG = decltype(ng)::value;
+    constexpr bool E = decltype(ext)::value;
+    if (fast)
+      shell_fp64_kernel<NG, false, true><<<blocks, threads, 0, s>>>(P);
+    else
+      shell_fp64_kernel<NG, E, false><<<blocks, threads, 0, s>>>(P);
+  });
+}
+
+}  // namespace hxg

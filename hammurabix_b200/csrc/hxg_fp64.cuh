@@ -1,0 +1,437 @@
+// hxg_fp64.cuh -- the FP64 (parity) shell kernel: every value of the ray, the
+// fields, the emissivity and the sums in FP64.
+//
+// Speed.  The sample loop is bound by the FP64 pipe, so it is written for few
+// FP64 instructions at unchanged precision:
+//   - everything is expressed in the frame turned by the ray's azimuth, where
+//     the ray stays at constant Y: the position is X(d), Y, z(d), the field is
+//     (B_X, B_Y, B_z), B_par = st B_X + ct B_z, and the sky components are
+//     -(ct B_X - st B_z) and -B_Y; no Cartesian position or versor products;
+//   - grid coordinates are linear in the distance, one FMA each, split with
+//     one round-down add; the 8 corners are summed with weights, each record
+//     read with one 32-byte load (two 16-byte loads each take the L1 data
+//     stage twice as long);
+//   - a ray's window is trimmed with the cut test itself, so the samples
+//     between its ends need no test (without an inner radius), and the window,
+//     not the whole ray, is cut into the chunks of a pixel's lanes;
+//   - divisions by model parameters are products with their reciprocals, the
+//     remaining functions come from hxg_math64.cuh, two exponentials of one
+//     product are one, and launch constants multiply the sums once;
+//   - |B_perp|^2 of CRE index 3 needs neither root nor power, and the angle's
+//     cos 2ipa, sin 2ipa never divide by |B_perp|^2.
+//
+// Measured (B200, two passes over Nside 64/128/256 to 30 kpc on 256^3 grids):
+// 34.4 ms before these, 19.4 ms with the sample arithmetic, 14.4 ms with the
+// window cut into chunks and the coefficients as constant operands (30 of 32
+// lanes active against 20), 13.1 ms with quarter warps of neighbouring rays at
+// 128 x 5, 11.6 ms with 32-byte record loads.  A sample is 161 FP64
+// instructions, 80 clocks of an SM's FP64 pipes, and about as many of its L1
+// data stage (8 records of 32 bytes for each of 32 lanes); the two together
+// bound the loop, each about 60 % busy.
+#pragma once
+
+#include "hxg_integrate.cuh"
+
+// Launch shape of the FP64 shell kernels: threads per block and the resident
+// blocks per SM their register allocation must allow.  128 x 5 (96 registers,
+// 20 warps, no spills with one grid) runs the case above in 11.6 ms against
+// 12.4 ms at 128 x 4 and 12.1 ms at 128 x 6 (80 registers, spills).
+#ifndef HXG_FP64_THREADS
+#define HXG_FP64_THREADS 128
+#endif
+#ifndef HXG_FP64_MIN_BLOCKS
+#define HXG_FP64_MIN_BLOCKS 5
+#endif
+
+namespace hxg {
+
+// Sample range [i0, i1) of chunk c of a ray: the ray window (ray_window) trimmed
+// with the cut test itself, |pos| <= r_max and z_min <= z <= z_max
+// (integrator.cc:179-182), then cut into equal parts.  Ball and slab are
+// convex, so the passing samples are one run and need no further test (but
+// for an inner radius).  Equal parts of the window, not of the whole ray: a
+// warp's chunks end together, where parts of the ray left the outer chunks of
+// the outer shells empty.  The adjoint takes the same ranges.
+__device__ __forceinline__ void chunk_range64(const ShellLaunch &P, const double u[3], int c,
+                                              int &i0, int &i1) {
+  const auto pass = [&](long long i) {
+    const double d = fma((double)i + 0.5, P.delta, P.d_start);
+    const double px = fma(u[0], d, P.obs[0]), py = fma(u[1], d, P.obs[1]),
+                 pz = fma(u[2], d, P.obs[2]);
+    const double len = sqrt(px * px + py * py + pz * pz);
+    return !(len > P.gc_r_max || pz < P.gc_z_min || pz > P.gc_z_max);
+  };
+  long long lo, hi, slo_unused, shi_unused;
+  ray_window(P, u[0], u[1], u[2], lo, hi, slo_unused, shi_unused);
+  while (lo < hi && !pass(lo)) ++lo;
+  while (hi > lo && !pass(hi - 1)) --hi;
+  // sample indices fit 32 bits (checked on the host)
+  const long long n = max(hi - lo, 0ll);
+  i0 = (int)(lo + ((n * c) >> P.log2_chunks));
+  i1 = (int)(lo + ((n * (c + 1)) >> P.log2_chunks));
+}
+
+// The ray's coordinates in a grid group, g(d) = g0 + gv d per axis, and the
+// samples [ga, gb) of [i0, i1) that lie inside its box (0 < g < n - 1 on
+// every axis, breg.cc:34-54): the slab intersections, widened by two samples
+// and trimmed with the test itself (the rounded g(d) is monotone in d).
+struct GridRay64 {
+  double g0[3], gv[3];
+  int ga, gb;
+};
+__device__ __forceinline__ void grid_ray64(const ShellLaunch &P, const DevGridGroup &G,
+                                           const double u[3], int i0, int i1, GridRay64 &R) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    R.g0[k] = (P.obs[k] - G.lo[k]) * G.scale[k];
+    R.gv[k] = u[k] * G.scale[k];
+  }
+  grid_window(P, G, R.g0, R.gv, i0, i1, R.ga, R.gb);
+  const auto in = [&](int i) {
+    const double d = fma((double)i + 0.5, P.delta, P.d_start);
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double g = fma(R.gv[k], d, R.g0[k]);
+      ok = ok && g > 0. && g < G.gmax[k];
+    }
+    return ok;
+  };
+  while (R.ga < R.gb && !in(R.ga)) ++R.ga;
+  while (R.gb > R.ga && !in(R.gb - 1)) --R.gb;
+}
+
+// Cell and fraction of a grid coordinate 0 < g < 2^31: adding 2^52 rounded
+// down leaves floor(g) in the low word.
+__device__ __forceinline__ void cell64(double g, int &cell, double &frac) {
+  const double t = __dadd_rd(g, kC64.floor52);
+  cell = __double2loint(t);
+  frac = g - (t - kC64.floor52);
+}
+
+// One voxel record (32 bytes, aligned to 32) in one load.
+__device__ __forceinline__ void load_rec32(const double2 *p, double2 &a, double2 &b) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
+      : "l"(p));
+}
+
+// Trilinear sample of the FP64 records at distance d (breg.cc:58-96): the 8
+// corner records summed with their weights.  out = bx, by, bz, n_e.
+__device__ __forceinline__ void trilinear64(const DevGridGroup &G, const GridRay64 &R, double d,
+                                            double out[4]) {
+  int cx, cy, cz;
+  double fx, fy, fz;
+  cell64(fma(R.gv[0], d, R.g0[0]), cx, fx);
+  cell64(fma(R.gv[1], d, R.g0[1]), cy, fy);
+  cell64(fma(R.gv[2], d, R.g0[2]), cz, fz);
+  // record indices fit 32 bits (the host refuses larger grids)
+  const unsigned i00 =
+      ((unsigned)cx * (unsigned)G.ny + (unsigned)cy) * (unsigned)G.nz + (unsigned)cz;
+  const double2 *p = reinterpret_cast<const double2 *>(G.rec) + 2 * (size_t)i00;
+  const size_t sy = 2 * (size_t)G.nz, sx = sy * (size_t)G.ny;
+  const double ex = 1. - fx, ey = 1. - fy, ez = 1. - fz;
+  const double w4[4] = {ex * ey, ex * fy, fx * ey, fx * fy};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double2 *q = p + (k & 1 ? sy : 0) + (k & 2 ? sx : 0);
+    double2 a0, a1, b0, b1;
+    load_rec32(q, a0, a1);
+    load_rec32(q + 2, b0, b1);
+    const double wa = w4[k] * ez, wb = w4[k] * fz;
+    if (k == 0) {
+      out[0] = wa * a0.x;
+      out[1] = wa * a0.y;
+      out[2] = wa * a1.x;
+      out[3] = wa * a1.y;
+    } else {
+      out[0] = fma(wa, a0.x, out[0]);
+      out[1] = fma(wa, a0.y, out[1]);
+      out[2] = fma(wa, a1.x, out[2]);
+      out[3] = fma(wa, a1.y, out[3]);
+    }
+    out[0] = fma(wb, b0.x, out[0]);
+    out[1] = fma(wb, b0.y, out[1]);
+    out[2] = fma(wb, b1.x, out[2]);
+    out[3] = fma(wb, b1.y, out[3]);
+  }
+}
+
+// CRE_ana spatial profile exp((R0 - r)/r0) sech^2(z/z0) (cre_ana.cc:11-63):
+//   = e^((R0 - r)/r0 - 2|z|/z0) (2 / (1 + t))^2, t = e^(-2|z|/z0).
+template <bool kRange>
+__device__ __forceinline__ double cre_ana_prof64(const FastModels &F, double r, double az) {
+  const double a = az * F.cre64_2iz0;
+  const double t = exp64<kRange>(-a);
+  const double e = exp64<kRange>(fma(F.cre64_R0 - r, F.cre64_ir0, -a));
+  const double i = rcp64(fma(t, 0.5, 0.5));
+  return e * (i * i);
+}
+
+// |B_perp|^pe of the constant-index emissivity, b2 = |B_perp|^2 in units of
+// 2^-40 G^2 (k_t and k_p carry the unit), so that the logarithm stays small.
+// With an exponent e = (index + 1)/2 above 0 the reference's A^e |B_perp| at
+// zero field is inf * 0.
+__device__ __forceinline__ double bperp_pow64(const ShellLaunch &P, double b2) {
+  if (P.em_pe == 1.) return sqrt(b2);
+  if (b2 == 0.) return P.em_pe < 1. ? nan("") : 0.;
+  return exp64<true>(0.5 * P.em_pe * log(b2));
+}
+
+// Warp gw of shell launch P (32/C pixels, C lanes each) for the NF frequency
+// passes of Fq.  All 32 lanes of the warp call it with the same gw.  kFast:
+// the launch's models satisfy fast_models and exp_ok (the other models and the
+// exponentials' range checks compiled out).
+template <int NG, bool kExt, int NF, bool kFast>
+__device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF> &Fq,
+                                          long long gw, int lane) {
+  const int C = P.chunks;
+  // the warp's 32/C pixels side by side, chunk after chunk: the lanes of a
+  // load's quarter warp are neighbouring rays at the same distance, which
+  // share cache lines
+  const int S = 32 >> P.log2_chunks;
+  const int seg = lane & (S - 1);
+  const int c = lane >> (5 - P.log2_chunks);
+  const Hpx h = hpx_make((uint64_t)P.nside);
+  const unsigned long long nest =
+      shard_nest(P, (unsigned long long)gw * S + seg);
+  const bool valid = nest < h.npix;
+  uint64_t ring = 0;
+  bool live = false;
+  if (valid) {
+    ring = hpx_nest2ring(h, nest);
+    live = (P.mask == nullptr) || (P.mask[ring] != 0);
+  }
+  double dm = 0., fd = 0., si[NF], sq[NF], su[NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) si[f] = sq[f] = su[f] = 0.;
+  if (live) {
+    double th, ph;
+    hpx_pix2ang(h, ring, th, ph);
+    double inner = 0.;
+    if (P.fdmap != nullptr) {
+      const Hpx hf = hpx_make((uint64_t)P.nside_fdmap);
+      inner = hpx_interpolate(hf, P.fdmap, th, ph);
+    }
+    if (NF == 1 && P.ck_inner != nullptr && c == 0) P.ck_inner[ring] = inner;
+    const double st = sin(th), ct = cos(th), sp = sin(ph), cp = cos(ph);
+    // los_versor (integrator.cc:268-272)
+    const double u[3] = {cp * st, sp * st, ct};
+    const DevModels &M = P.models;
+    const FastModels &F = P.fast;
+    const double oz = P.obs[2];
+    // the observer in the frame turned by the ray's azimuth
+    const double oX = fma(cp, P.obs[0], sp * P.obs[1]);
+    const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
+    // r^2 along the ray is X^2 + YY; never 0, so that 1/r is finite
+    const double YY = fma(Y, Y, 1e-280);
+    const double csY = F.sp_cos_s * Y, ssY = F.sp_sin_s * Y;
+    const bool fast_b = M.breg == kBregSpiral;
+    const bool fast_t = M.tereg == kTeregExpdisk;
+    const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
+    const bool slow_t = !kFast && M.tereg != kTeregNone && !fast_t;
+    const bool cre_ana = kFast || M.cre == kCreAna;
+    // Faraday phase in quarter turns: q0 + quarter_k * (FD sum), per pass
+    double q0[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      q0[f] = Fq.inner[f] ? inner * Fq.quarter_i[f] : 0.;
+    const bool pe2 = P.em_const && P.em_pe == 2.;
+    double sdm = 0., sfd = 0., last_index = nan(""), gt = P.em_gt, gp = P.em_gp;
+    int i0, i1;
+    chunk_range64(P, u, c, i0, i1);
+    GridRay64 R;
+    if (NG == 1) grid_ray64(P, P.groups[0], u, i0, i1, R);
+    double x = (double)i0 + 0.5;
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i, x += 1.) {
+      const double d = fma(x, P.delta, P.d_start);
+      const double z = fma(ct, d, oz);
+      const double X = fma(st, d, oX);
+      const double r2 = fma(X, X, YY);
+      double p3[3] = {0., 0., 0.};
+      if (!kFast || NG > 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p3[k] = fma(u[k], d, P.obs[k]);
+        // an inner radius can split a ray's passing samples in two runs
+        if (!kFast && P.gc_r_min > 0. && sqrt(r2 + z * z) < P.gc_r_min) continue;
+      }
+      // the grid first: its loads return while the models are evaluated
+      double g[4] = {0., 0., 0., 0.};
+      if (NG == 1) {
+        if ((unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) trilinear64(P.groups[0], R, d, g);
+      } else if (NG > 1) {
+        double b3[3] = {0., 0., 0.};
+        CellCache<double> cc;
+#pragma unroll 1
+        for (int k = 0; k < P.ngroups; ++k)
+          sample_group<double, false>(P.groups[k], p3[0], p3[1], p3[2], cc, b3, g[3]);
+        g[0] = b3[0];
+        g[1] = b3[1];
+        g[2] = b3[2];
+      }
+      const double ir = rsqrt64(r2), r = r2 * ir;
+      const double az = fabs(z);
+      double bX = 0., bY = 0., bz = 0., te = 0.;
+      // positive doubles compare like integers, off the FP64 pipe
+      if (fast_b && __double_as_longlong(r2) >= __double_as_longlong(F.rc2_lo) &&
+          __double_as_longlong(r2) <= __double_as_longlong(F.rc2_hi)) {
+        const double a = exp64<!kFast>(fma(F.sp_rsun - r, F.sp_irs, -(az * F.sp_ihs))) * ir;
+        bX = a * fma(F.sp_sin_s, X, -csY);
+        bY = a * fma(F.sp_cos_s, X, ssY);
+      }
+      if (fast_t) te = F.ex_n0 * exp64<!kFast>(-fma(r, F.ex_irn, az * F.ex_ihn));
+      if (slow_b) {
+        const V3<double> B = breg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
+        bX = fma(cp, B.x, sp * B.y);
+        bY = fma(cp, B.y, -(sp * B.x));
+        bz = B.z;
+      }
+      if (slow_t) te = tereg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
+      if (NG > 0) {
+        bX = fma(cp, g[0], fma(sp, g[1], bX));
+        bY = fma(cp, g[1], fma(-sp, g[0], bY));
+        bz += g[2];
+        te += g[3];
+      }
+      // n_e clamped at 0 (integrator.cc:201); NaN stays NaN
+      if (__double2hiint(te) < 0) te *= 0.;
+      sdm += te;
+      sfd = fma(te, fma(st, bX, ct * bz), sfd);
+      if (P.do_sync) {
+        // B_perp on the sky basis: |B_perp|^2 = xv^2 + yv^2, cos 2ipa =
+        // (xv^2 - yv^2) / |B_perp|^2, sin 2ipa = 2 xv yv / |B_perp|^2
+        // (integrator.cc:257-265); both signs of (xv, yv) give the same
+        const double xv = bY, yv = fma(ct, bX, -(st * bz));
+        const double x2 = xv * xv;
+        const double rr = fma(yv, yv, x2), cc2 = fma(-yv, yv, x2), hs2 = xv * yv;
+        double wt[NF], wpc[NF], wps[NF];
+        constexpr int NW = kFast ? 1 : NF;
+        bool shared_w = true;
+        if (kExt && M.cre == kCreGrid) {
+          // spectral integral over the CRE grid (integrator.cc:288-330,
+          // 357-400); the host fuses no CRE-grid pass
+          double jt, jp;
+          cre_grid_j(P.ext->cre, p3[0], p3[1], p3[2], sqrt(rr), jt, jp);
+          const double inv = rr > 0. ? 1. / rr : 0.;
+          wt[0] = jt;
+          wpc[0] = rr > 0. ? jp * cc2 * inv : jp;
+          wps[0] = 2. * jp * hs2 * inv;
+        } else {
+          const double prof = cre_ana ? cre_ana_prof64<!kFast>(F, r, az)
+                                      : cre_profile<double>(M, p3[0], p3[1], p3[2], p3);
+          if (pe2) {
+            wt[0] = prof * rr;
+            wpc[0] = prof * cc2;
+            wps[0] = (prof + prof) * hs2;
+          } else {
+            double wp[NF];
+            if (kFast || P.em_const) {
+              wt[0] = wp[0] = prof * bperp_pow64(P, rr * 0x1p40);
+            } else {
+              shared_w = false;
+              const double index = cre_index<double>(M, p3[0], p3[1], p3[2]);
+              if (index != last_index) {
+                gt = tgamma(-0.25 * index + 19. / 12.) * tgamma(-0.25 * index - 1. / 12.);
+                gp = tgamma(-0.25 * index + 7. / 12.) * tgamma(-0.25 * index - 1. / 12.);
+                last_index = index;
+              }
+              const double bper = sqrt(rr);
+#pragma unroll
+              for (int f = 0; f < NW; ++f) {
+                const double base = prof * bper * pow(Fq.a_s[f] / bper, 0.5 * (index + 1));
+                wt[f] = base * gt / (1. - index);
+                wp[f] = base * gp;
+              }
+            }
+            // ipa of a zero B_perp is 0 (atan2(0, 0)): cos 2ipa = 1
+            const double inv = rr > 0. ? rcp64(rr) : 0.;
+#pragma unroll
+            for (int f = 0; f < NW; ++f) {
+              if (f > 0 && shared_w) break;
+              wpc[f] = rr > 0. ? wp[f] * (cc2 * inv) : wp[f];
+              wps[f] = 2. * wp[f] * (hs2 * inv);
+            }
+          }
+        }
+        if (shared_w) {
+#pragma unroll
+          for (int f = 1; f < NF; ++f) {
+            wt[f] = wt[0];
+            wpc[f] = wpc[0];
+            wps[f] = wps[0];
+          }
+        }
+        si[0] += wt[0];
+        if (!kFast) {
+#pragma unroll
+          for (int f = 1; f < NF; ++f) si[f] += wt[f];
+        }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+          double sf, cf;
+          sincos_quarter(fma(Fq.quarter_k[f], sfd, q0[f]), sf, cf);
+          sq[f] = fma(cf, wpc[f], fma(-sf, wps[f], sq[f]));
+          su[f] = fma(sf, wpc[f], fma(cf, wps[f], su[f]));
+        }
+      }
+    }
+    dm = sdm * P.delta;
+    fd = sfd * P.fd_fore * P.delta;
+    // I is one sum for all passes of the constant-index models
+    const double s0 = si[0];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      si[f] = (kFast ? s0 : si[f]) * Fq.k_t[f];
+      sq[f] *= Fq.k_p[f];
+      su[f] *= Fq.k_p[f];
+    }
+  }
+  // adjoint checkpoint (one pass): the chunk's FD and local-frame Q, U
+  // before the chunk combination
+  if (NF == 1 && P.ck != nullptr && live) {
+    const unsigned long long ci = nest * (unsigned long long)C + c;
+    P.ck[3 * ci] = fd;
+    P.ck[3 * ci + 1] = sq[0];
+    P.ck[3 * ci + 2] = su[0];
+  }
+  combine_chunks_nf<NF>(P, Fq, c, dm, fd, si, sq, su, S);
+  if (live && c == 0) {
+    if (P.do_dm) P.out[0][ring] = dm;
+    if (P.do_fd || P.do_sync) P.out[1][ring] = fd;
+    if (P.do_sync) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        Fq.out[f][0][ring] = si[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+        Fq.out[f][1][ring] = sq[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+        Fq.out[f][2][ring] = su[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+      }
+    }
+  } else if (valid && !live && c == 0) {
+    // masked pixel: every observable is zero (integrator.cc:63-67, 98-115)
+    if (P.do_dm) P.out[0][ring] = 0.;
+    if (P.do_fd || P.do_sync) P.out[1][ring] = 0.;
+    if (P.do_sync) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        Fq.out[f][0][ring] = Fq.out[f][1][ring] = Fq.out[f][2][ring] = 0.;
+    }
+  }
+}
+
+// One frequency pass: the pass's constants from its launch block.
+template <int NG, bool kExt, bool kFast>
+__device__ __forceinline__ void fp64_tile(const ShellLaunch &P, long long gw, int lane) {
+  FreqSet<1> Fq;
+  freq_of_launch(P, Fq);
+  fp64_tile<NG, kExt, 1, kFast>(P, Fq, gw, lane);
+}
+
+template <int NG, bool kExt, bool kFast>
+__global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MIN_BLOCKS)
+shell_fp64_kernel(const ShellLaunch P) {
+  fp64_tile<NG, kExt, kFast>(P, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                             threadIdx.x & 31);
+}
+
+}  // namespace hxg

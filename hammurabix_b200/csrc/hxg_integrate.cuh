@@ -14,13 +14,15 @@
 
 #include "hxg_common.cuh"
 #include "hxg_fields.cuh"
+#include "hxg_math64.cuh"
 
 namespace hxg {
 
 constexpr int kMaxGroups = 4;
 
-// FP32C evaluation of the spiral B and exponential n_e models (FP64, kpc
-// and 2^-20 G, reciprocals precomputed).
+// The spiral B, exponential n_e and CRE_ana models as the sample loops
+// evaluate them: reciprocals and launch constants precomputed, in FP64 and the
+// working units of the form (FP32C: kpc and 2^-20 G).
 struct FastModels {
   double sp_b0, sp_irs, sp_crs, sp_ihs;  // amplitude, 1/r_s, r_sun/r_s, 1/h_s
   double sp_sin, sp_cos;                 // sin, cos of the pitch angle
@@ -29,6 +31,9 @@ struct FastModels {
   // r_sun/r_s + ln|b0| and ln n0, the sign of b0 into sp_*_s
   double sp_crs_l, ex_ln0;
   double sp_sin_s, sp_cos_s;             // sign(b0) sin, sign(b0) cos
+                                         // (FP64 form: b0 sin, b0 cos)
+  double sp_rsun;                        // r_sun
+  double cre64_R0, cre64_ir0, cre64_2iz0;  // CRE_ana: R0, 1/r0, 2/|z0|
   float sp_sinf_s, sp_cosf_s;            // the same in FP32
   // launch constants in the types the sample loop uses, so that the loop
   // reads them as operands instead of converting them
@@ -71,9 +76,11 @@ struct ShellLaunch {
   double em_n0u;             // j0 * gamma0^-index(observer) * unit
   double em_qe3, em_den_t, em_den_p, em_anum, em_3qe;
   double em_gt, em_gp;       // Gamma products at the constant index
-  // FP32C scales (applied in FP64 after the sums)
+  // scales applied in FP64 after the sums
   double k_t, k_p, k_dm;     // I, Q/U and DM scale factors
-  double phase_k;            // 2 lambda^2 * fd_fore (per FP64 FD-sum unit)
+  double phase_k;            // 2 lambda^2 * FD per unit of the FD sum
+  double quarter_k;          // the same in quarter turns (FP64 form), and
+  double quarter_i;          // quarter turns per unit of the inner-shell FD
   double a_s;                // A * |B_perp| in 2^-20 G (variable-index path)
   double em_pe;              // exponent of |B_perp| (constant index, FP32C)
   DevModels models;
@@ -83,7 +90,8 @@ struct ShellLaunch {
   // before the chunk combination, per pixel the inner-shell FD; null = off
   double *ck;
   double *ck_inner;
-  FastModels fast;  // FP32C only
+  FastModels fast;
+  int exp_ok;            // every exponent of the FastModels is below 680 in size
   const ExtModels *ext;  // Jaffe / JF12 / YMW16 blocks (device), or null
 };
 
@@ -130,13 +138,32 @@ __host__ __device__ inline bool fast_models(const ShellLaunch &P) {
 template <int NF>
 struct FreqSet {
   double lambda2[NF];   // (c/nu)^2
-  double phase_k[NF];   // 2 lambda^2 * fd_fore (per FP64 FD-sum unit)
+  double phase_k[NF];   // 2 lambda^2 * FD per unit of the FD sum
+  double quarter_k[NF]; // the same in quarter turns (FP64 form)
+  double quarter_i[NF]; // quarter turns per unit of the inner-shell FD
   double k_t[NF], k_p[NF];
   double tc_a[NF], tc_b[NF];
   double a_s[NF];       // A * |B_perp| scale of the variable-index emissivity
   int inner[NF];        // 1: the pass reads the inner-shell FD (its do_fd)
   double *out[NF][3];   // I, Q, U shell maps
 };
+
+// One pass's constants from its launch block.
+__device__ __forceinline__ void freq_of_launch(const ShellLaunch &P, FreqSet<1> &Fq) {
+  Fq.lambda2[0] = P.lambda2;
+  Fq.phase_k[0] = P.phase_k;
+  Fq.quarter_k[0] = P.quarter_k;
+  Fq.quarter_i[0] = P.quarter_i;
+  Fq.k_t[0] = P.k_t;
+  Fq.k_p[0] = P.k_p;
+  Fq.tc_a[0] = P.tc_a;
+  Fq.tc_b[0] = P.tc_b;
+  Fq.a_s[0] = P.a_s;
+  Fq.inner[0] = 1;
+  Fq.out[0][0] = P.out[2];
+  Fq.out[0][1] = P.out[3];
+  Fq.out[0][2] = P.out[4];
+}
 
 // NESTED index of the shard's local pixel `local`: local pixels run through
 // the shard's blocks in order.
@@ -196,6 +223,31 @@ __device__ __forceinline__ void ray_window(const ShellLaunch &P, double ux,
   }
 }
 
+// Sample range [ga, gb) of [i0, i1) in which the ray can be inside the grid
+// box 0 < g < n - 1 on every axis (from the slab intersections in FP64,
+// widened by two samples; the caller's own test decides each sample).
+__device__ __forceinline__ void grid_window(const ShellLaunch &P, const DevGridGroup &G,
+                                            const double g0[3], const double gv[3],
+                                            int i0, int i1, int &ga, int &gb) {
+  double da = -1e300, db = 1e300;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (gv[k] != 0.) {
+      const double t0 = -g0[k] / gv[k], t1 = (G.gmax[k] - g0[k]) / gv[k];
+      da = fmax(da, fmin(t0, t1));
+      db = fmin(db, fmax(t0, t1));
+    } else if (!(g0[k] > 0. && g0[k] < G.gmax[k])) {
+      db = -1e300;
+    }
+  }
+  ga = i1;
+  gb = i1;
+  if (!(da <= db)) return;
+  const double xa = (da - P.d_start) / P.delta - 0.5, xb = (db - P.d_start) / P.delta - 0.5;
+  ga = (int)fmin(fmax(floor(xa) - 2., (double)i0), (double)i1);
+  gb = (int)fmin(fmax(ceil(xb) + 3., (double)ga), (double)i1);
+}
+
 // Kahan-compensated FP32 accumulator.
 struct KahanF {
   float s, c;
@@ -235,35 +287,43 @@ __device__ __forceinline__ double shfl_xor_d(double v, int o) {
 
 // Combine the C chunk partial sums of each pixel: exclusive FD prefix over
 // the chunks, rotation of each chunk's Q/U by 2*lambda^2*prefix, butterfly
-// reduction inside the C-lane segment.  All 32 lanes participate.
-__device__ __forceinline__ void combine_chunks(const ShellLaunch &P, int c,
-                                               double rot_k, double &dm,
-                                               double &fd, double &si,
-                                               double &sq, double &su) {
+// reduction over the pixel's C lanes, `stride` lanes apart.  All 32 lanes
+// participate.
+template <int NF>
+__device__ __forceinline__ void combine_chunks_nf(const ShellLaunch &P, const FreqSet<NF> &Fq,
+                                                  int c, double &dm, double &fd, double si[NF],
+                                                  double sq[NF], double su[NF],
+                                                  int stride = 1) {
   const int C = P.chunks;
   if (C == 1) return;
   // inclusive scan of fd within the segment
   double incl = fd;
   for (int o = 1; o < C; o <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, incl, o);
+    const double v = __shfl_up_sync(0xffffffffu, incl, o * stride);
     if (c >= o) incl += v;
   }
-  double excl = __shfl_up_sync(0xffffffffu, incl, 1);
+  double excl = __shfl_up_sync(0xffffffffu, incl, stride);
   if (c == 0) excl = 0.;
-  if (P.do_sync && c > 0) {
-    double sr, cr;
-    sincos(rot_k * excl, &sr, &cr);
-    const double q = sq * cr - su * sr;
-    const double u = sq * sr + su * cr;
-    sq = q;
-    su = u;
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    if (P.do_sync && c > 0) {
+      double sr, cr;
+      sincos(2. * Fq.lambda2[f] * excl, &sr, &cr);
+      const double q = sq[f] * cr - su[f] * sr;
+      const double u = sq[f] * sr + su[f] * cr;
+      sq[f] = q;
+      su[f] = u;
+    }
   }
   for (int o = C >> 1; o > 0; o >>= 1) {
-    dm += shfl_xor_d(dm, o);
-    fd += shfl_xor_d(fd, o);
-    si += shfl_xor_d(si, o);
-    sq += shfl_xor_d(sq, o);
-    su += shfl_xor_d(su, o);
+    dm += shfl_xor_d(dm, o * stride);
+    fd += shfl_xor_d(fd, o * stride);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      si[f] += shfl_xor_d(si[f], o * stride);
+      sq[f] += shfl_xor_d(sq[f], o * stride);
+      su[f] += shfl_xor_d(su[f], o * stride);
+    }
   }
 }
 
@@ -281,181 +341,6 @@ __device__ __forceinline__ void ipa2(T xv, T yv, T &c2, T &s2) {
     c2 = T(1);
     s2 = T(0);
   }
-}
-
-// ===================================================================
-// FP64 parity form
-// ===================================================================
-// Warp gw of shell launch P (32/C pixels, C lanes each).  All 32 lanes of
-// the warp call it with the same gw.  kFast: the launch's models satisfy
-// fast_models (the same arithmetic, the other models compiled out).
-template <int NG, bool kCache, bool kExt, bool kFast = false>
-__device__ __forceinline__ void fp64_tile(const ShellLaunch &P, long long gw,
-                                          int lane) {
-  const int C = P.chunks;
-  const int seg = lane >> P.log2_chunks;
-  const int c = lane & (C - 1);
-  const Hpx h = hpx_make((uint64_t)P.nside);
-  const unsigned long long nest =
-      shard_nest(P, (unsigned long long)gw * (32 >> P.log2_chunks) + seg);
-  const bool valid = nest < h.npix;
-  uint64_t ring = 0;
-  bool live = false;
-  if (valid) {
-    ring = hpx_nest2ring(h, nest);
-    live = (P.mask == nullptr) || (P.mask[ring] != 0);
-  }
-  double dm = 0., fd = 0., si = 0., sq = 0., su = 0.;
-  const double rot_k = 2. * P.lambda2;
-  if (live) {
-    double th, ph;
-    hpx_pix2ang(h, ring, th, ph);
-    double inner = 0.;
-    if (P.fdmap != nullptr) {
-      const Hpx hf = hpx_make((uint64_t)P.nside_fdmap);
-      inner = hpx_interpolate(hf, P.fdmap, th, ph);
-    }
-    if (P.ck_inner != nullptr && c == 0) P.ck_inner[ring] = inner;
-    const double st = sin(th), ct = cos(th), sp = sin(ph), cp = cos(ph);
-    // los_versor (integrator.cc:268-272)
-    const double ux = cp * st, uy = sp * st, uz = ct;
-    // spherical unit vectors of sync_ipa (integrator.cc:260-262)
-    const double etx = ct * cp, ety = ct * sp, etz = -st;
-    const double epx = -sp, epy = cp;
-    const DevModels &M = P.models;
-    CellCache<double> cache;
-    cache.key = -1;
-    double last_index = nan(""), gt = P.em_gt, gp = P.em_gp;
-    long long wlo, whi, slo, shi;
-    ray_window(P, ux, uy, uz, wlo, whi, slo, shi);
-    const long long i0 = max((P.step * c) >> P.log2_chunks, wlo);
-    const long long i1 = min((P.step * (c + 1)) >> P.log2_chunks, whi);
-    for (long long i = i0; i < i1; ++i) {
-      const double d = P.d_start + ((double)i + 0.5) * P.delta;
-      const double px = ux * d + P.obs[0];
-      const double py = uy * d + P.obs[1];
-      const double pz = uz * d + P.obs[2];
-      if (i < slo || i >= shi) {
-        const double len = sqrt(px * px + py * py + pz * pz);
-        if (len < P.gc_r_min || len > P.gc_r_max || pz < P.gc_z_min ||
-            pz > P.gc_z_max)
-          continue;
-      }
-      const double p3[3] = {px, py, pz};
-      V3<double> B{0., 0., 0.};
-      double te = 0.;
-      if (kFast) {
-        if (M.breg == kBregSpiral) B = breg_spiral<double>(M, px, py, pz, p3);
-        if (M.tereg == kTeregExpdisk) te = tereg_expdisk<double>(M, px, py, pz);
-      } else {
-        B = breg_model_x<kExt>(M, P.ext, px, py, pz, p3);
-        te = tereg_model_x<kExt>(M, P.ext, px, py, pz, p3);
-      }
-      if (NG > 0) {
-        double b3[3] = {B.x, B.y, B.z};
-#pragma unroll 1
-        for (int g = 0; g < (NG == 1 ? 1 : P.ngroups); ++g)
-          sample_group<double, kCache>(P.groups[g], px, py, pz, cache, b3, te);
-        B.x = b3[0];
-        B.y = b3[1];
-        B.z = b3[2];
-      }
-      te *= (double)(te > 0.);
-      const double bpar = B.x * ux + B.y * uy + B.z * uz;
-      const double cx = B.y * uz - B.z * uy;
-      const double cy = B.z * ux - B.x * uz;
-      const double cz = B.x * uy - B.y * ux;
-      const double bper = sqrt(cx * cx + cy * cy + cz * cz);
-      if (P.do_dm) dm += te * P.delta;
-      if (P.do_fd || P.do_sync) fd += te * bpar * P.fd_fore * P.delta;
-      if (P.do_sync) {
-        double jtot, jpol;
-        if (kExt && M.cre == kCreGrid) {
-          // spectral integral over the CRE grid (integrator.cc:288-330, 357-400)
-          double jt, jp;
-          cre_grid_j(P.ext->cre, px, py, pz, bper, jt, jp);
-          jtot = jt * P.delta * P.i2bt;
-          jpol = jp * P.delta * P.i2bt;
-        } else {
-          double index = P.em_index;
-          if (!kFast && !P.em_const) {
-            index = cre_index<double>(M, px, py, pz);
-            if (index != last_index) {
-              gt = tgamma(-0.25 * index + 19. / 12.) * tgamma(-0.25 * index - 1. / 12.);
-              gp = tgamma(-0.25 * index + 7. / 12.) * tgamma(-0.25 * index - 1. / 12.);
-              last_index = index;
-            }
-          }
-          const double fn = P.em_n0u * (kFast ? cre_profile_ana<double>(M, px, py, pz)
-                                              : cre_profile<double>(M, px, py, pz, p3));
-          const double absb = fabs(bper);
-          const double A = P.em_anum / (P.em_3qe * absb);
-          double Ae;
-          if (P.em_const && P.em_pow_kind == 1)
-            Ae = 1. / A;
-          else if (P.em_const && P.em_pow_kind == 2)
-            Ae = 1.;
-          else
-            Ae = pow(A, 0.5 * (index + 1));
-          const double den_t = P.em_const ? P.em_den_t
-                                          : 4. * cgs::pi * cgs::mec2 * (1. - index);
-          const double norm_t = fn * 1.73205081 * P.em_qe3 * absb / den_t;
-          const double norm_p = fn * 1.73205081 * P.em_qe3 * absb / P.em_den_p;
-          jtot = norm_t * (Ae * gt) * P.delta * P.i2bt;
-          jpol = norm_p * (Ae * gp) * P.delta * P.i2bt;
-        }
-        si += jtot;
-        double c2, s2;
-        ipa2<double>(-(epx * B.x + epy * B.y), -(etx * B.x + ety * B.y + etz * B.z),
-                     c2, s2);
-        double sf, cf;
-        sincos(2. * ((inner + fd) * P.lambda2), &sf, &cf);
-        sq += (cf * c2 - sf * s2) * jpol;
-        su += (sf * c2 + cf * s2) * jpol;
-      }
-    }
-  }
-  if (P.ck != nullptr && live) {
-    const unsigned long long ci = nest * (unsigned long long)C + c;
-    P.ck[3 * ci] = fd;
-    P.ck[3 * ci + 1] = sq;
-    P.ck[3 * ci + 2] = su;
-  }
-  combine_chunks(P, c, rot_k, dm, fd, si, sq, su);
-  if (live && c == 0) {
-    if (P.do_dm) P.out[0][ring] = dm;
-    if (P.do_fd || P.do_sync) P.out[1][ring] = fd;
-    if (P.do_sync) {
-      P.out[2][ring] = si * P.tc_a * P.tc_a / P.tc_b;
-      P.out[3][ring] = sq * P.tc_a * P.tc_a / P.tc_b;
-      P.out[4][ring] = su * P.tc_a * P.tc_a / P.tc_b;
-    }
-  } else if (valid && !live && c == 0) {
-    // masked pixel: every observable is zero (integrator.cc:63-67, 98-115)
-    if (P.do_dm) P.out[0][ring] = 0.;
-    if (P.do_fd || P.do_sync) P.out[1][ring] = 0.;
-    if (P.do_sync) P.out[2][ring] = P.out[3][ring] = P.out[4][ring] = 0.;
-  }
-}
-
-// Launch shape of the FP64 shell kernel: threads per block and the resident
-// blocks per SM its register allocation must allow.  128 x 7 (72
-// registers, 28 warps per SM) ran the config-3 FP64 passes in 490.6 ms
-// against 492.7 ms at 128 x 6, 494.0 ms at 256 x 3, 499.5 ms at 256 x 4,
-// 513 ms at 128 x 5, 566 ms at 128 x 4 and 574 ms with the compiler's own
-// choice at 256 threads (104 registers, 16 warps).
-#ifndef HXG_FP64_THREADS
-#define HXG_FP64_THREADS 128
-#endif
-#ifndef HXG_FP64_MIN_BLOCKS
-#define HXG_FP64_MIN_BLOCKS 7
-#endif
-
-template <int NG, bool kCache, bool kExt, bool kFast = false>
-__global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MIN_BLOCKS)
-shell_fp64_kernel(const ShellLaunch P) {
-  fp64_tile<NG, kCache, kExt, kFast>(P, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                              threadIdx.x & 31);
 }
 
 }  // namespace hxg

@@ -2,11 +2,10 @@
 // packing, and the instantiations of the shell-integration kernels.
 #include <cuda_runtime.h>
 
-#include <type_traits>
-
 #include "hxg_adjoint.cuh"
 #include "hxg_adjoint32.cuh"
 #include "hxg_batch.cuh"
+#include "hxg_dispatch.cuh"
 #include "hxg_fp32c.cuh"
 #include "hxg_integrate.cuh"
 #include "hxg_internal.h"
@@ -448,40 +447,17 @@ cudaError_t launch_pack(cudaStream_t s, bool fp32, uint64_t n, void *rec,
   return cudaGetLastError();
 }
 
-// The kernels are instantiated per grid-group count (0, 1, up to
-// kMaxGroups) and per use of the Jaffe / JF12 / YMW16 blocks.
-template <typename F>
-static cudaError_t by_shape(int ngroups, bool ext, F &&f) {
-  const auto g = [&](auto ng) {
-    if (ext)
-      f(ng, std::true_type{});
-    else
-      f(ng, std::false_type{});
-  };
-  if (ngroups == 0)
-    g(std::integral_constant<int, 0>{});
-  else if (ngroups == 1)
-    g(std::integral_constant<int, 1>{});
-  else
-    g(std::integral_constant<int, 4>{});
-  return cudaGetLastError();
-}
-
 cudaError_t launch_shell(cudaStream_t s, bool fp32, const ShellLaunch &P,
                          unsigned blocks, unsigned threads) {
+  if (!fp32) return launch_shell64(s, P, blocks, threads);
   const bool fast = fast_models(P);
   return by_shape(P.ngroups, P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ext)::value;
-    if (fp32 && fast)
+    if (fast)
       shell_fp32c_kernel<NG, false, true><<<blocks, threads, 0, s>>>(P);
-    else if (fp32)
-      shell_fp32c_kernel<NG, E, false><<<blocks, threads, 0, s>>>(P);
-    else if (fast)
-      shell_fp64_kernel<NG, false, false, true><<<blocks, threads, 0, s>>>(P);
     else
-      shell_fp64_kernel<decltype(ng)::value, false, decltype(ext)::value>
-          <<<blocks, threads, 0, s>>>(P);
+      shell_fp32c_kernel<NG, E, false><<<blocks, threads, 0, s>>>(P);
   });
 }
 

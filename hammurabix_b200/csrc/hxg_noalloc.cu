@@ -18,7 +18,7 @@
 #include <mutex>
 
 #include "../../include/hxg.h"
-#include "hxg_integrate.cuh"
+#include "hxg_fp64.cuh"
 #include "hxg_internal.h"
 
 namespace hxg {
