@@ -1683,9 +1683,6 @@ int hxg_write_grid_device(hxg_handle *h, const hxg_obs_t *o, double *d_dm,
 
 namespace {
 
-// Whether passes o[0..n) can share one shell traversal: FP32C form, the
-// same observer, shells, radial step, limits and mask switch, synchrotron on
-// in every pass, and no CRE grid (its emissivity depends on the frequency).
 // Passes o[0..n) with synchrotron output and the same observer, shells,
 // radial step, limits and mask switch: one traversal can serve them all.
 bool same_traversal(const hxg_obs_t *o, int n) {
@@ -1705,10 +1702,13 @@ bool same_traversal(const hxg_obs_t *o, int n) {
   return true;
 }
 
-// Whether passes o[0..n) of the handle's models can share one traversal:
-// FP32C form, no CRE grid (its emissivity depends on the frequency).
+// Whether passes o[0..n) of the handle's models can share one traversal: no
+// CRE grid (its emissivity depends on the frequency).  The FP64 form with
+// checkpointing on runs them one by one: the last one's checkpoint stays
+// usable by the adjoint.
 bool fusable(const hxg_handle *h, const hxg_obs_t *o, int n) {
-  if (h->precision != HXG_FP32C || n < 2 || h->models.cre == HXG_CRE_GRID) return false;
+  if (n < 2 || h->models.cre == HXG_CRE_GRID) return false;
+  if (h->precision == HXG_FP64 && h->checkpoint) return false;
   return same_traversal(o, n);
 }
 
@@ -1771,7 +1771,8 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
   P.log2_chunks = hpx_ilog2((uint64_t)C);
   if (local == 0) return HXG_OK;
   const uint64_t warps = (local + (32 / C) - 1) / (32 / C);
-  const unsigned threads = HXG_FP32C_MULTI_THREADS;
+  const bool fp32 = h->precision == HXG_FP32C;
+  const unsigned threads = fp32 ? HXG_FP32C_MULTI_THREADS : HXG_FP64_THREADS;
   const unsigned blocks = (unsigned)((warps * 32 + threads - 1) / threads);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->timing) {
@@ -1779,7 +1780,7 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
     HXG_CK(cudaEventCreate(&e1));
     HXG_CK(cudaEventRecord(e0, h->stream));
   }
-  HXG_CK(launch_shell_multi(h->stream, P, NF, &Fq, blocks, threads));
+  HXG_CK(launch_shell_multi(h->stream, fp32, P, NF, &Fq, blocks, threads));
   ++h->launch_count;
   if (h->timing) {
     HXG_CK(cudaEventRecord(e1, h->stream));
@@ -1877,13 +1878,22 @@ int hxg_write_grid_multi(hxg_handle *h, int npass, const hxg_obs_t *obs, double 
   while (k < npass) {
     const int left = npass - k;
     const int nf = left >= 3 && fusable(h, obs + k, 3) ? 3 : (left >= 2 && fusable(h, obs + k, 2) ? 2 : 1);
+    const auto one = [&](int q) {
+      double *const *m = d_outs + 5 * q;
+      return hxg_write_grid_device(h, obs + q, m[0], m[1], m[2], m[3], m[4]);
+    };
     if (nf == 3)
       st = write_fused<3>(h, obs + k, d_outs + 5 * k);
     else if (nf == 2)
       st = write_fused<2>(h, obs + k, d_outs + 5 * k);
-    else {
-      double *const *m = d_outs + 5 * k;
-      st = hxg_write_grid_device(h, obs + k, m[0], m[1], m[2], m[3], m[4]);
+    else
+      st = one(k);
+    // the shell maps of several passes are too much for the device (they
+    // are allocated before any launch): one by one
+    if (st == HXG_ERR_OOM && nf > 1 && h->precision == HXG_FP64) {
+      (void)cudaGetLastError();
+      st = HXG_OK;
+      for (int q = k; q < k + nf && st == HXG_OK; ++q) st = one(q);
     }
     if (st != HXG_OK) return st;
     k += nf;
@@ -1992,7 +2002,7 @@ int hxg_shell_integrate_multi_device(hxg_handle *h, int npass, const hxg_obs_t *
     if (o[f].do_fd && fd_pass < 0) fd_pass = f;
   }
   if (!d_tmp_fd) return fail(h, HXG_ERR_INVALID, "the shell FD map is always written");
-  if (!fusable(h, o, npass))
+  if (h->precision != HXG_FP32C || !fusable(h, o, npass))
     return fail(h, HXG_ERR_UNSUPPORTED, "these passes cannot share a traversal");
   const uint64_t npix = npix_of(o[0].nside_shell[shell]);
   double *tmp_iqu[3][3];

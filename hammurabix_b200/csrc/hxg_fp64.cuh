@@ -18,7 +18,9 @@
 //     remaining functions come from hxg_math64.cuh, two exponentials of one
 //     product are one, and launch constants multiply the sums once;
 //   - |B_perp|^2 of CRE index 3 needs neither root nor power, and the angle's
-//     cos 2ipa, sin 2ipa never divide by |B_perp|^2.
+//     cos 2ipa, sin 2ipa never divide by |B_perp|^2;
+//   - up to three frequency passes of one geometry share the traversal: a
+//     further pass adds its phase and Q, U sums, 23 FP64 instructions.
 //
 // Measured (B200, two passes over Nside 64/128/256 to 30 kpc on 256^3 grids):
 // 34.4 ms before these, 19.4 ms with the sample arithmetic, 14.4 ms with the
@@ -41,6 +43,12 @@
 #endif
 #ifndef HXG_FP64_MIN_BLOCKS
 #define HXG_FP64_MIN_BLOCKS 5
+#endif
+// The fused kernels: three passes over Nside 128-1024 on 512^3 grids 91.7 ms
+// (205.3 ms pass by pass; 94.4 at 128 x 4, 95.4 at 128 x 6), two passes over
+// the case above 6.8 ms (7.2, 7.1).
+#ifndef HXG_FP64_MULTI_MIN_BLOCKS
+#define HXG_FP64_MULTI_MIN_BLOCKS 5
 #endif
 
 namespace hxg {
@@ -432,6 +440,14 @@ __global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MIN_BLOCKS)
 shell_fp64_kernel(const ShellLaunch P) {
   fp64_tile<NG, kExt, kFast>(P, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                              threadIdx.x & 31);
+}
+
+// NF frequency passes in one traversal of the shell.
+template <int NG, bool kExt, int NF, bool kFast>
+__global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MULTI_MIN_BLOCKS)
+shell_fp64_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
+  fp64_tile<NG, kExt, NF, kFast>(P, Fq, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                                 threadIdx.x & 31);
 }
 
 }  // namespace hxg

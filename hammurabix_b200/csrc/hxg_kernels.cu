@@ -461,8 +461,9 @@ cudaError_t launch_shell(cudaStream_t s, bool fp32, const ShellLaunch &P,
   });
 }
 
-cudaError_t launch_shell_multi(cudaStream_t s, const ShellLaunch &P, int nf, const void *fq,
-                               unsigned blocks, unsigned threads) {
+cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, int nf,
+                               const void *fq, unsigned blocks, unsigned threads) {
+  if (!fp32) return launch_shell64_multi(s, P, nf, fq, blocks, threads);
   const bool fast = fast_models(P);
   return by_shape(P.ngroups, P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
