@@ -755,6 +755,9 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     F.cre_2iz0_l2 = float(2. * cgs::log2e / D.cre_z0);
     F.cre_R0_l2 = float(2. + D.cre_R0 * cgs::log2e / D.cre_r0);
     F.pe = float(P.em_pe);
+    P.fast_ok = (D.breg != kBregSpiral ||
+                 std::isfinite(F.sp_irs + F.sp_ihs + F.sp_crs_l)) &&
+                (D.tereg != kTeregExpdisk || std::isfinite(F.ex_irn + F.ex_ihn + F.ex_ln0));
   } else {
     P.fd_fore = fdfore;
     P.phase_k = 2. * P.lambda2 * fdfore * delta;
@@ -767,13 +770,16 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     F.cre64_R0 = D.cre_R0;
     F.cre64_ir0 = 1. / D.cre_r0;
     F.cre64_2iz0 = 2. / std::fabs(D.cre_z0);
-    // largest exponents inside the cuts: r, |z| <= gc_r_max
+    // largest exponents inside the cuts
     const double rm = P.gc_r_max + D.sp_rsun;
-    const auto below = [](double a) { return std::fabs(a) < 680.; };
-    P.exp_ok = (D.breg != kBregSpiral || below(rm * (std::fabs(F.sp_irs) + std::fabs(F.sp_ihs)))) &&
-               (D.tereg != kTeregExpdisk ||
-                below(rm * (std::fabs(F.ex_irn) + std::fabs(F.ex_ihn)))) &&
-               (D.cre != kCreAna || below(rm * (std::fabs(F.cre64_ir0) + F.cre64_2iz0)));
+    const double zm =
+        std::min(P.gc_r_max, std::max(std::fabs(P.gc_z_min), std::fabs(P.gc_z_max)));
+    const auto below = [&](double ir, double iz) {
+      return std::fabs(rm * ir) + std::fabs(zm * iz) < 680.;
+    };
+    P.fast_ok = (D.breg != kBregSpiral || below(F.sp_irs, F.sp_ihs)) &&
+                (D.tereg != kTeregExpdisk || below(F.ex_irn, F.ex_ihn)) &&
+                (D.cre != kCreAna || below(F.cre64_ir0, F.cre64_2iz0));
   }
   // grid groups
   P.ngroups = (int)h->groups.size();
@@ -2977,7 +2983,7 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
     uint64_t step;
     if ((st = build_launch(h, E.models, E.obs, 0, L, step)) != HXG_OK) return bail(st);
     L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) : nullptr;
-    b->fast = b->fast && hxg::fast_models(L) && (b->fp32 || L.exp_ok);
+    b->fast = b->fast && hxg::fast_models(L) && L.fast_ok;
   }
   int per_sm = 0;
   cudaError_t ce = hxg::batch_level_occupancy(b->fp32, b->ngroups, b->ext_any, b->fast, &per_sm);

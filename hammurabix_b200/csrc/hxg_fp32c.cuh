@@ -114,15 +114,22 @@ __device__ __forceinline__ void trilinear_f32(const float4 *rec, int ny,
 // relative; the rounding of ln2/64 times k adds below 6e-14): a systematic
 // error that moves the Faraday phase at 0.408 GHz, thousands of radians,
 // by under 1e-9 rad.
+// kFast (finite launch constants, so a is no NaN): the bound is taken on the
+// high word alone.  With that, the integer bound of 1/r's argument and the
+// coefficients as constant operands (the same values and bits), three passes
+// over Nside 128-1024 on 512^3 grids went from 59.1 to 57.4 ms.
+template <bool kFast = false>
 __device__ __forceinline__ double exp_tab(double a) {
-  const double kMagic = 6755399441055744.0;  // 1.5 * 2^52
-  a = fmax(a, -700.);
-  const double t = fma(a, 92.33248261689366, kMagic);   // 64 / ln2
+  if (kFast)
+    a = __hiloint2double((int)min((unsigned)__double2hiint(a), 0xC085E000u), __double2loint(a));
+  else
+    a = fmax(a, -700.);
+  const double t = fma(a, kC64.k64_ln2, kC64.magic);
   const int k = __double2loint(t);
-  const double kd = t - kMagic;
-  const double r = fma(-kd, 0.010830424696249145, a);   // ln2 / 64
-  double p = 4.1666666666666664e-02;                    // 1/4!
-  p = fma(p, r, 1.6666666666666666e-01);                // 1/3!
+  const double kd = t - kC64.magic;
+  const double r = fma(-kd, kC64.ln2_64_hi, a);
+  double p = kC64.e4;                                   // 1/4!
+  p = fma(p, r, kC64.e3);                               // 1/3!
   p = fma(p, r, 0.5);
   p = fma(p, r, 1.0);
   p = fma(p, r, 1.0);
@@ -348,7 +355,9 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
         const double rc2 = fma(px, px, py * py);
         // on the z axis r is 1e-150 instead of 0 (y finite; the spiral is
         // cut there)
-        const double rc2m = fmax(rc2, 1e-300);
+        const double rc2m =
+            kFast ? __hiloint2double(max(__double2hiint(rc2), 0x01A56E1F), __double2loint(rc2))
+                  : fmax(rc2, 1e-300);
         const double y = rsqrt_fd(rc2m);
         const double r = rc2m * y;
         rcf = float(r);
@@ -356,7 +365,7 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
           // kFast: b0 exp(a) = sign(b0) exp(a + ln|b0|), the sign in ss, cs
           const double sarg =
               fma(-r, F.sp_irs, fma(-fabs(pz), F.sp_ihs, kFast ? F.sp_crs_l : F.sp_crs));
-          const double ay = kFast ? exp_tab(sarg) * y : F.sp_b0 * exp_tab(sarg) * y;
+          const double ay = kFast ? exp_tab<true>(sarg) * y : F.sp_b0 * exp_tab(sarg) * y;
           bp_d = ay * fma(K1, d, K0);
           const float ayf = float(ay);
           bxr = ayf * (spf * xf - cpf * yf);
@@ -364,7 +373,7 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
         }
         if (fast_t) {
           if (kFast)  // n0 exp(a) = exp(a + ln n0), n0 > 0
-            te_d = exp_tab(fma(-r, F.ex_irn, fma(-fabs(pz), F.ex_ihn, F.ex_ln0)));
+            te_d = exp_tab<true>(fma(-r, F.ex_irn, fma(-fabs(pz), F.ex_ihn, F.ex_ln0)));
           else
             te_d = F.ex_n0 * exp_tab(-fma(r, F.ex_irn, fabs(pz) * F.ex_ihn));
         }

@@ -15,7 +15,7 @@ static int shape64(const ShellLaunch &P) {
 
 cudaError_t launch_shell64(cudaStream_t s, const ShellLaunch &P, unsigned blocks,
                            unsigned threads) {
-  const bool fast = fast_models(P) && P.exp_ok;
+  const bool fast = fast_models(P) && P.fast_ok;
   return by_shape(shape64(P), P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ext)::value;
@@ -28,7 +28,7 @@ cudaError_t launch_shell64(cudaStream_t s, const ShellLaunch &P, unsigned blocks
 
 cudaError_t launch_shell64_multi(cudaStream_t s, const ShellLaunch &P, int nf, const void *fq,
                                  unsigned blocks, unsigned threads) {
-  const bool fast = fast_models(P) && P.exp_ok;
+  const bool fast = fast_models(P) && P.fast_ok;
   return by_shape(shape64(P), P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ext)::value;

@@ -188,7 +188,7 @@ __device__ __forceinline__ double bperp_pow64(const ShellLaunch &P, double b2) {
 
 // Warp gw of shell launch P (32/C pixels, C lanes each) for the NF frequency
 // passes of Fq.  All 32 lanes of the warp call it with the same gw.  kFast:
-// the launch's models satisfy fast_models and exp_ok (the other models and the
+// the launch's models satisfy fast_models and fast_ok (the other models and the
 // exponentials' range checks compiled out).
 template <int NG, bool kExt, int NF, bool kFast>
 __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF> &Fq,

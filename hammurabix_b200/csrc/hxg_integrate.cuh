@@ -91,7 +91,9 @@ struct ShellLaunch {
   double *ck;
   double *ck_inner;
   FastModels fast;
-  int exp_ok;            // every exponent of the FastModels is below 680 in size
+  // FP64 form: every exponent of the FastModels is below 680 in size; FP32C:
+  // its constants are finite (the kFast instantiations need it)
+  int fast_ok;
   const ExtModels *ext;  // Jaffe / JF12 / YMW16 blocks (device), or null
 };
 

@@ -450,7 +450,7 @@ cudaError_t launch_pack(cudaStream_t s, bool fp32, uint64_t n, void *rec,
 cudaError_t launch_shell(cudaStream_t s, bool fp32, const ShellLaunch &P,
                          unsigned blocks, unsigned threads) {
   if (!fp32) return launch_shell64(s, P, blocks, threads);
-  const bool fast = fast_models(P);
+  const bool fast = fast_models(P) && P.fast_ok;
   return by_shape(P.ngroups, P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ext)::value;
@@ -464,7 +464,7 @@ cudaError_t launch_shell(cudaStream_t s, bool fp32, const ShellLaunch &P,
 cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, int nf,
                                const void *fq, unsigned blocks, unsigned threads) {
   if (!fp32) return launch_shell64_multi(s, P, nf, fq, blocks, threads);
-  const bool fast = fast_models(P);
+  const bool fast = fast_models(P) && P.fast_ok;
   return by_shape(P.ngroups, P.ext != nullptr, [&](auto ng, auto ext) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ext)::value;
