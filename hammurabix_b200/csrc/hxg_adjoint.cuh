@@ -8,7 +8,8 @@
 // with warp shuffles, the pixel totals Q, U and each chunk's prefix, so a
 // single forward-ordered sweep suffices: the reverse-accumulated phase
 // sensitivity S_i = sum_{k >= i} dL/dchi_k equals
-// 2 (gU (Q - Q_{<i}) - gQ (U - U_{<i})).
+// 2 (gU (Q - Q_{<i}) - gQ (U - U_{<i})), one running sum since gQ, gU are
+// constant along a ray.
 //
 // Per sample i (symbols of integrator.cc:173-226):
 //   t_i   = n_e B_par K dl           (Faraday-depth term, K = fd_forefactor)
@@ -18,6 +19,13 @@
 //   J ~ |B_perp|^(1-e), e = (index+1)/2  ->  dJ/d|B_perp| = (1-e) J / |B_perp|
 //   dipa/dB = (-x e_theta + y e_phi) / (x^2 + y^2),  y = -e_theta.B,
 //   x = -e_phi.B
+//
+// The sample is fp64_tile's, in the frame turned by the ray's azimuth (there
+// u = (st, 0, ct), e_theta = (ct, 0, -st), e_phi = (0, 1, 0)); its reverse
+// adds about 90 FP64 instructions to the forward's 161.  The grid-record
+// gradient of a cell is summed in registers while the ray stays in it and
+// flushed with 32 atomic adds at record offsets (the cell index is the offset
+// of its first corner: no divisions).
 #pragma once
 
 #include "hxg_fp64.cuh"
@@ -40,35 +48,37 @@ struct AdjointLaunch {
   int want_j0;              // 1 when the CRE normalisation gradient is wanted
 };
 
-__device__ __forceinline__ void flush_cell(double *grad_rec, long long key,
-                                           int ny, int nz, double acc[8][4]) {
-  if (key < 0 || grad_rec == nullptr) return;
-  const long long nyz = (long long)ny * nz;
-  const long long xl = key / nyz;
-  const long long yl = (key - xl * nyz) / nz;
-  const long long zl = key - xl * nyz - yl * nz;
+constexpr unsigned kNoCell = 0xFFFFFFFFu;
+
+// Adds the accumulators of the cell whose corner 000 is record `key` into the
+// record gradient and clears them.
+template <typename T>
+__device__ __forceinline__ void flush_cell(double *grad_rec, unsigned key, unsigned ny,
+                                           unsigned nz, T acc[8][4]) {
+  if (key == kNoCell) return;
+  const unsigned nyz = ny * nz;
 #pragma unroll
   for (int dx = 0; dx < 2; ++dx)
 #pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
+    for (int dy = 0; dy < 2; ++dy) {
+      double *p = grad_rec + 4 * (size_t)(key + dx * nyz + dy * nz);
 #pragma unroll
-      for (int dz = 0; dz < 2; ++dz) {
-        const int k = dx * 4 + dy * 2 + dz;
-        const long long idx = (xl + dx) * nyz + (yl + dy) * nz + (zl + dz);
-        double *p = grad_rec + 4 * idx;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (acc[k][c] != 0.) atomicAdd(p + c, acc[k][c]);
-          acc[k][c] = 0.;
-        }
+      for (int k = 0; k < 8; ++k) {
+        T &a = acc[dx * 4 + dy * 2 + (k >> 2)][k & 3];
+        atomicAdd(p + k, (double)a);
+        a = T(0);
       }
+    }
 }
 
 // Launch shape of the adjoint shell kernel (threads per block, resident
 // blocks per SM its register allocation must allow).  128 x 3 (168
 // registers, 12 warps per SM; the per-cell gradient accumulators take 64)
-// ran the config-4 adjoint in 49.9 ms against 52.4 ms at 128 x 4 (128
-// registers, more spills) and 62.2 ms at 256 x 1 (254 registers, 8 warps).
+// runs forward, loss and backward on 256^3 grids, Nside 64/128/256, in 23.0 ms
+// against 25.4 ms at 128 x 4 (128 registers, spills) and 26.1 ms at 128 x 2;
+// 44.7 ms with the kernel before, which evaluated the sample with the
+// reference's operations, divided 64-bit indices in every flush and had
+// 1670 warp instructions a sample (FP64 pipe 37 % busy).
 #ifndef HXG_ADJ_THREADS
 #define HXG_ADJ_THREADS 128
 #endif
@@ -168,180 +178,187 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
         for (int k = 0; k < 4; ++k) atomicAdd(A.g_fdmap + pix[k], g_inner * w[k] / wtot);
     }
     const double st = sin(th), ct = cos(th), sp = sin(ph), cp = cos(ph);
-    const double ux = cp * st, uy = sp * st, uz = ct;
-    const double etx = ct * cp, ety = ct * sp, etz = -st;
-    const double epx = -sp, epy = cp;
+    const double u[3] = {cp * st, sp * st, ct};
     const DevModels &M = P.models;
+    const FastModels &F = P.fast;
+    const double oz = P.obs[2];
+    const double oX = fma(cp, P.obs[0], sp * P.obs[1]);
+    const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
+    const double YY = fma(Y, Y, 1e-280);
+    const double csY = F.sp_cos_s * Y, ssY = F.sp_sin_s * Y;
+    const bool fast_b = M.breg == kBregSpiral;
+    const bool fast_t = M.tereg == kTeregExpdisk;
+    const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
+    const bool slow_t = !kFast && M.tereg != kTeregNone && !fast_t;
+    const bool pe2 = P.em_const && P.em_pe == 2.;
+    // dL/d(the sample's weights): the launch scales folded in
+    const double gIk = gI * P.k_t, gQk = gQ * P.k_p, gUk = gU * P.k_p;
+    const double K = P.fd_fore * P.delta, gdmd = gdm * P.delta;
+    // gfd + lambda^2 S_i, running: S starts at the chunk's own
+    double gtt = fma(2. * l2, gU * (Qp - Qrun) - gQ * (Up - Urun), gfd);
+    if (!P.do_sync) gtt = gfd;
+    const double l2x2 = 2. * l2;
+    // Faraday phase in quarter turns: inner + Fc + the running chunk FD (the
+    // sample's own term included)
+    const double q0 = (inner + Fc) * P.quarter_i;
     double acc[8][4];
 #pragma unroll
     for (int k = 0; k < 8; ++k)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[k][q] = 0.;
-    long long acc_key = -1;
+    unsigned acc_key = kNoCell;
     double gt = P.em_gt, gpp = P.em_gp, last_index = nan("");
-    double fdl = 0.;  // running FD of this chunk
-    const double u3[3] = {ux, uy, uz};
+    double sfd = 0.;  // running FD of this chunk (FD-sum units)
     int i0, i1;
-    chunk_range64(P, u3, c, i0, i1);
-    for (int i = i0; i < i1; ++i) {
-      const double d = P.d_start + ((double)i + 0.5) * P.delta;
-      const double px = ux * d + P.obs[0];
-      const double py = uy * d + P.obs[1];
-      const double pz = uz * d + P.obs[2];
-      if (!kFast && P.gc_r_min > 0. && sqrt(px * px + py * py + pz * pz) < P.gc_r_min) continue;
-      const double p3[3] = {px, py, pz};
-      V3<double> Breg{0., 0., 0.};
-      double tereg = 0.;
-      if (kFast) {
-        if (M.breg == kBregSpiral) Breg = breg_spiral<double>(M, px, py, pz, p3);
-        if (M.tereg == kTeregExpdisk) tereg = tereg_expdisk<double>(M, px, py, pz);
-      } else {
-        Breg = breg_model_x<kExt>(M, P.ext, px, py, pz, p3);
-        tereg = tereg_model_x<kExt>(M, P.ext, px, py, pz, p3);
+    chunk_range64(P, u, c, i0, i1);
+    GridRay64 R;
+    if (NG == 1) grid_ray64(P, P.groups[0], u, i0, i1, R);
+    double x = (double)i0 + 0.5;
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i, x += 1.) {
+      const double d = fma(x, P.delta, P.d_start);
+      const double z = fma(ct, d, oz);
+      const double X = fma(st, d, oX);
+      const double r2 = fma(X, X, YY);
+      double p3[3] = {0., 0., 0.};
+      if (!kFast) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p3[k] = fma(u[k], d, P.obs[k]);
+        if (P.gc_r_min > 0. && sqrt(r2 + z * z) < P.gc_r_min) continue;
       }
-      double b3[3] = {Breg.x, Breg.y, Breg.z};
-      double te = tereg;
-      bool in_grid = false;
-      int xl = 0, yl = 0, zl = 0;
-      double xd = 0., yd = 0., zd = 0.;
+      double g[4] = {0., 0., 0., 0.};
+      Cell64 W;
+      W.key = kNoCell;
+      if (NG == 1 && (unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) {
+        cell_of64(P.groups[0], R, d, W);
+        trilinear64(P.groups[0], W, g);
+      }
+      const double ir = rsqrt64(r2), r = r2 * ir;
+      const double az = fabs(z);
+      double sX = 0., sY = 0., bX = 0., bY = 0., bz = 0., te_d = 0.;
+      if (fast_b && __double_as_longlong(r2) >= __double_as_longlong(F.rc2_lo) &&
+          __double_as_longlong(r2) <= __double_as_longlong(F.rc2_hi)) {
+        const double a = exp64<!kFast>(fma(F.sp_rsun - r, F.sp_irs, -(az * F.sp_ihs))) * ir;
+        sX = a * fma(F.sp_sin_s, X, -csY);
+        sY = a * fma(F.sp_cos_s, X, ssY);
+      }
+      bX = sX;
+      bY = sY;
+      if (fast_t) te_d = F.ex_n0 * exp64<!kFast>(-fma(r, F.ex_irn, az * F.ex_ihn));
+      double te = te_d;
+      if (slow_b) {
+        const V3<double> B = breg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
+        bX = fma(cp, B.x, sp * B.y);
+        bY = fma(cp, B.y, -(sp * B.x));
+        bz = B.z;
+      }
+      if (slow_t) te = tereg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
       if (NG > 0) {
-        const DevGridGroup &G = P.groups[0];
-        if (grid_coords(G, px, py, pz, xl, yl, zl, xd, yd, zd)) {
-          in_grid = true;
-          CellCache<double> cc;
-          fill_cell<double>(G, xl, yl, zl, cc);
-          double out[4];
-          trilinear<double>(cc, xd, yd, zd, out);
-          b3[0] += out[0];
-          b3[1] += out[1];
-          b3[2] += out[2];
-          te += out[3];
-        }
+        bX = fma(cp, g[0], fma(sp, g[1], bX));
+        bY = fma(cp, g[1], fma(-sp, g[0], bY));
+        bz += g[2];
+        te += g[3];
       }
-      const double te_raw = te;
-      te *= (double)(te > 0.);
-      const double bx = b3[0], by = b3[1], bz = b3[2];
-      const double bpar = bx * ux + by * uy + bz * uz;
-      const double cx = by * uz - bz * uy, cy = bz * ux - bx * uz,
-                   cz = bx * uy - by * ux;
-      const double bper = sqrt(cx * cx + cy * cy + cz * cz);
-      const double t = te * bpar * P.fd_fore * P.delta;
-      fdl += t;
-      double g_te = gdm * P.delta;
-      double g_bpar = 0., g_bper = 0., g_ipa = 0.;
-      double xv = 0., yv = 0.;
-      double jt = 0., jp = 0., e = 0.;
+      const bool te_on = te > 0.;
+      if (!te_on) te *= 0.;
+      const double bpar = fma(st, bX, ct * bz);
+      sfd = fma(te, bpar, sfd);
+      double g_te = gdmd, g_bpar = 0., g_th = 0., g_ph = 0.;
       if (P.do_fd || P.do_sync) {
-        double gtt = gfd;
+        // phase sensitivity of the samples k >= i, the sample's own included
+        const double gk = gtt * K;
         if (P.do_sync) {
-          double index = P.em_index;
-          if (!kFast && !P.em_const) {
-            index = cre_index<double>(M, px, py, pz);
-            if (index != last_index) {
-              gt = tgamma(-0.25 * index + 19. / 12.) * tgamma(-0.25 * index - 1. / 12.);
-              gpp = tgamma(-0.25 * index + 7. / 12.) * tgamma(-0.25 * index - 1. / 12.);
-              last_index = index;
+          const double xv = bY, yv = fma(ct, bX, -(st * bz));
+          const double x2 = xv * xv;
+          const double rr = fma(yv, yv, x2), cc2 = fma(-yv, yv, x2), hs2 = xv * yv;
+          const double irr = rr > 1e-300 ? rcp64(rr) : 0.;
+          double wt, wpc, wps, pe = P.em_pe;
+          const double prof = (kFast || M.cre == kCreAna)
+                                  ? cre_ana_prof64<!kFast>(F, r, az)
+                                  : cre_profile<double>(M, p3[0], p3[1], p3[2], p3);
+          if (pe2) {
+            wt = prof * rr;
+            wpc = prof * cc2;
+            wps = (prof + prof) * hs2;
+          } else {
+            double wp;
+            if (kFast || P.em_const) {
+              wt = wp = prof * bperp_pow64(P, rr * 0x1p40);
+            } else {
+              const double index = cre_index<double>(M, p3[0], p3[1], p3[2]);
+              if (index != last_index) {
+                gt = tgamma(-0.25 * index + 19. / 12.) * tgamma(-0.25 * index - 1. / 12.);
+                gpp = tgamma(-0.25 * index + 7. / 12.) * tgamma(-0.25 * index - 1. / 12.);
+                last_index = index;
+              }
+              const double bper = sqrt(rr), e = 0.5 * (index + 1);
+              const double base = prof * bper * pow(P.a_s / bper, e);
+              wt = base * gt / (1. - index);
+              wp = base * gpp;
+              pe = 1. - e;
             }
+            wpc = rr > 0. ? wp * (cc2 * irr) : wp;
+            wps = 2. * wp * (hs2 * irr);
           }
-          e = 0.5 * (index + 1);
-          const double fn = P.em_n0u * (kFast ? cre_profile_ana<double>(M, px, py, pz)
-                                              : cre_profile<double>(M, px, py, pz, p3));
-          const double absb = fabs(bper);
-          const double Aa = P.em_anum / (P.em_3qe * absb);
-          double Ae;
-          if (P.em_const && P.em_pow_kind == 1)
-            Ae = 1. / Aa;
-          else if (P.em_const && P.em_pow_kind == 2)
-            Ae = 1.;
-          else
-            Ae = pow(Aa, e);
-          const double den_t = P.em_const ? P.em_den_t
-                                          : 4. * cgs::pi * cgs::mec2 * (1. - index);
-          jt = fn * 1.73205081 * P.em_qe3 * absb / den_t * (Ae * gt) * P.delta * P.i2bt;
-          jp = fn * 1.73205081 * P.em_qe3 * absb / P.em_den_p * (Ae * gpp) * P.delta *
-               P.i2bt;
-          xv = -(epx * bx + epy * by);
-          yv = -(etx * bx + ety * by + etz * bz);
-          double c2, s2;
-          ipa2<double>(xv, yv, c2, s2);
           double sf, cf;
-          sincos(2. * ((inner + Fc + fdl) * l2), &sf, &cf);
-          const double cos2 = cf * c2 - sf * s2;
-          const double sin2 = sf * c2 + cf * s2;
-          // S_i: sensitivity of the loss to the phase of samples k >= i
-          const double Si = 2. * (gU * (Qp - Qrun) - gQ * (Up - Urun));
-          Qrun += jp * cos2;
-          Urun += jp * sin2;
-          gtt += l2 * Si;
-          const double gjt = gI, gjp = gQ * cos2 + gU * sin2;
-          g_ipa = 2. * jp * (gU * cos2 - gQ * sin2);
-          if (bper > 0.) g_bper = (gjt * jt + gjp * jp) * (1. - e) / bper;
-          if (A.want_j0) gp[7] += gjt * jt + gjp * jp;
+          sincos_quarter(fma(P.quarter_k, sfd, q0), sf, cf);
+          const double qi = fma(cf, wpc, -(sf * wps)), ui = fma(sf, wpc, cf * wps);
+          const double dG = fma(gUk, qi, -(gQk * ui));
+          gtt = fma(-l2x2, dG, gtt);
+          const double ej = fma(gIk, wt, fma(gQk, qi, gUk * ui));
+          if (A.want_j0) gp[7] += ej;
+          // |B_perp|^pe along B_perp, the angle across it
+          const double ke = ej * pe * irr, ki = 2. * dG * irr;
+          g_th = fma(ke, yv, ki * xv);
+          g_ph = fma(ke, xv, -(ki * yv));
         }
-        g_te += gtt * bpar * P.fd_fore * P.delta;
-        g_bpar = gtt * te * P.fd_fore * P.delta;
+        g_te = fma(gk, bpar, g_te);
+        g_bpar = gk * te;
       }
-      if (!(te_raw > 0.)) g_te = 0.;
-      // dL/dB
-      double gbx = g_bpar * ux, gby = g_bpar * uy, gbz = g_bpar * uz;
-      if (bper > 0.) {
-        const double k = g_bper / bper;
-        gbx += k * (bx - bpar * ux);
-        gby += k * (by - bpar * uy);
-        gbz += k * (bz - bpar * uz);
+      if (!te_on) g_te = 0.;
+      const double gX = fma(ct, g_th, st * g_bpar), gz = fma(ct, g_bpar, -(st * g_th));
+      // analytic-model parameter gradients (the constants after the loop);
+      // B = amp (sin(pitch - phi), cos(pitch - phi)), so dB/dpitch is B turned
+      // by -90 degrees
+      if (fast_b) {
+        const double gdotb = fma(gX, sX, g_ph * sY);
+        gp[0] += gdotb;
+        gp[1] += fma(gX, sY, -(g_ph * sX));
+        gp[2] = fma(gdotb, r - F.sp_rsun, gp[2]);
+        gp[3] = fma(gdotb, az, gp[3]);
       }
-      const double r2 = xv * xv + yv * yv;
-      if (g_ipa != 0. && r2 > 0.) {
-        const double k = g_ipa / r2;
-        gbx += k * (-xv * etx + yv * epx);
-        gby += k * (-xv * ety + yv * epy);
-        gbz += k * (-xv * etz);
-      }
-      // analytic-model parameter gradients
-      if (M.breg == kBregSpiral && (Breg.x != 0. || Breg.y != 0.)) {
-        const double r = sqrt(px * px + py * py);
-        const double gdotb = gbx * Breg.x + gby * Breg.y;
-        gp[0] += gdotb / M.sp_b0;
-        // B = amp (sin(pitch - phi), cos(pitch - phi)), so dB/dpitch is B
-        // turned by -90 degrees: (B_y, -B_x)
-        gp[1] += gbx * Breg.y - gby * Breg.x;
-        gp[2] += gdotb * (r - M.sp_rsun) / (M.sp_rs * M.sp_rs);
-        gp[3] += gdotb * fabs(pz) / (M.sp_hs * M.sp_hs);
-      }
-      if (M.tereg == kTeregExpdisk && tereg != 0.) {
-        const double r = sqrt(px * px + py * py);
-        gp[4] += g_te * tereg / M.tex_n0;
-        gp[5] += g_te * tereg * r / (M.tex_rs * M.tex_rs);
-        gp[6] += g_te * tereg * fabs(pz) / (M.tex_hs * M.tex_hs);
+      if (fast_t) {
+        const double gd = g_te * te_d;
+        gp[4] += gd;
+        gp[5] = fma(gd, r, gp[5]);
+        gp[6] = fma(gd, az, gp[6]);
       }
       // grid-record gradients, accumulated per cell
-      if (NG > 0 && in_grid && A.grad_rec != nullptr) {
-        const DevGridGroup &G = P.groups[0];
-        const long long key = (long long)xl * ((long long)G.ny * G.nz) +
-                              (long long)yl * G.nz + zl;
-        if (key != acc_key) {
-          flush_cell(A.grad_rec, acc_key, G.ny, G.nz, acc);
-          acc_key = key;
+      if (NG > 0 && W.key != kNoCell && A.grad_rec != nullptr) {
+        if (W.key != acc_key) {
+          flush_cell(A.grad_rec, acc_key, (unsigned)P.groups[0].ny, (unsigned)P.groups[0].nz,
+                     acc);
+          acc_key = W.key;
         }
-        const double wx[2] = {1. - xd, xd}, wy[2] = {1. - yd, yd},
-                     wz[2] = {1. - zd, zd};
+        const double gv[4] = {fma(cp, gX, -(sp * g_ph)), fma(sp, gX, cp * g_ph), gz, g_te};
 #pragma unroll
-        for (int dx = 0; dx < 2; ++dx)
+        for (int k = 0; k < 8; ++k) {
+          const double w = W.w4[k >> 1] * (k & 1 ? W.fz : W.ez);
 #pragma unroll
-          for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-            for (int dz = 0; dz < 2; ++dz) {
-              const double w = wx[dx] * wy[dy] * wz[dz];
-              const int k = dx * 4 + dy * 2 + dz;
-              acc[k][0] += w * gbx;
-              acc[k][1] += w * gby;
-              acc[k][2] += w * gbz;
-              acc[k][3] += w * g_te;
-            }
+          for (int q = 0; q < 4; ++q) acc[k][q] = fma(w, gv[q], acc[k][q]);
+        }
       }
     }
-    if (NG > 0)
-      flush_cell(A.grad_rec, acc_key, P.groups[0].ny, P.groups[0].nz, acc);
+    if (NG > 0 && A.grad_rec != nullptr)
+      flush_cell(A.grad_rec, acc_key, (unsigned)P.groups[0].ny, (unsigned)P.groups[0].nz, acc);
+    gp[0] = M.sp_b0 != 0. ? gp[0] / M.sp_b0 : 0.;
+    gp[2] *= F.sp_irs * F.sp_irs;
+    gp[3] *= F.sp_ihs * F.sp_ihs;
+    gp[4] = M.tex_n0 != 0. ? gp[4] / M.tex_n0 : 0.;
+    gp[5] *= F.ex_irn * F.ex_irn;
+    gp[6] *= F.ex_ihn * F.ex_ihn;
+    if (!fast_b) gp[0] = gp[1] = gp[2] = gp[3] = 0.;
+    if (!fast_t) gp[4] = gp[5] = gp[6] = 0.;
   }
   // parameter gradients: warp reduction, one atomic per warp and slot
   if (A.grad_par != nullptr) {

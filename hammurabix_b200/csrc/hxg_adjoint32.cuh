@@ -41,8 +41,6 @@
 
 namespace hxg {
 
-constexpr unsigned kNoCell = 0xFFFFFFFFu;
-
 // Adds the accumulators of the cell whose corner 000 is record `key` into
 // the FP64 record gradient and clears them.
 __device__ __forceinline__ void flush_cell32(double *grad_rec, unsigned key, unsigned ny,

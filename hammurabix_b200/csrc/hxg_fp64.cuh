@@ -124,29 +124,41 @@ __device__ __forceinline__ void load_rec32(const double2 *p, double2 &a, double2
       : "l"(p));
 }
 
-// Trilinear sample of the FP64 records at distance d (breg.cc:58-96): the 8
-// corner records summed with their weights.  out = bx, by, bz, n_e.
-__device__ __forceinline__ void trilinear64(const DevGridGroup &G, const GridRay64 &R, double d,
-                                            double out[4]) {
+// The cell of a sample: record index of its corner 000 (32 bits: the host
+// refuses larger grids), the (x, y) weights and the z weights.
+struct Cell64 {
+  unsigned key;
+  double w4[4], ez, fz;
+};
+__device__ __forceinline__ void cell_of64(const DevGridGroup &G, const GridRay64 &R, double d,
+                                          Cell64 &W) {
   int cx, cy, cz;
-  double fx, fy, fz;
+  double fx, fy;
   cell64(fma(R.gv[0], d, R.g0[0]), cx, fx);
   cell64(fma(R.gv[1], d, R.g0[1]), cy, fy);
-  cell64(fma(R.gv[2], d, R.g0[2]), cz, fz);
-  // record indices fit 32 bits (the host refuses larger grids)
-  const unsigned i00 =
-      ((unsigned)cx * (unsigned)G.ny + (unsigned)cy) * (unsigned)G.nz + (unsigned)cz;
-  const double2 *p = reinterpret_cast<const double2 *>(G.rec) + 2 * (size_t)i00;
+  cell64(fma(R.gv[2], d, R.g0[2]), cz, W.fz);
+  W.key = ((unsigned)cx * (unsigned)G.ny + (unsigned)cy) * (unsigned)G.nz + (unsigned)cz;
+  const double ex = 1. - fx, ey = 1. - fy;
+  W.ez = 1. - W.fz;
+  W.w4[0] = ex * ey;
+  W.w4[1] = ex * fy;
+  W.w4[2] = fx * ey;
+  W.w4[3] = fx * fy;
+}
+
+// Trilinear sample of the FP64 records (breg.cc:58-96): the 8 corner records
+// summed with their weights.  out = bx, by, bz, n_e.
+__device__ __forceinline__ void trilinear64(const DevGridGroup &G, const Cell64 &W,
+                                            double out[4]) {
+  const double2 *p = reinterpret_cast<const double2 *>(G.rec) + 2 * (size_t)W.key;
   const size_t sy = 2 * (size_t)G.nz, sx = sy * (size_t)G.ny;
-  const double ex = 1. - fx, ey = 1. - fy, ez = 1. - fz;
-  const double w4[4] = {ex * ey, ex * fy, fx * ey, fx * fy};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const double2 *q = p + (k & 1 ? sy : 0) + (k & 2 ? sx : 0);
     double2 a0, a1, b0, b1;
     load_rec32(q, a0, a1);
     load_rec32(q + 2, b0, b1);
-    const double wa = w4[k] * ez, wb = w4[k] * fz;
+    const double wa = W.w4[k] * W.ez, wb = W.w4[k] * W.fz;
     if (k == 0) {
       out[0] = wa * a0.x;
       out[1] = wa * a0.y;
@@ -267,7 +279,11 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
       // the grid first: its loads return while the models are evaluated
       double g[4] = {0., 0., 0., 0.};
       if (NG == 1) {
-        if ((unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) trilinear64(P.groups[0], R, d, g);
+        if ((unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) {
+          Cell64 W;
+          cell_of64(P.groups[0], R, d, W);
+          trilinear64(P.groups[0], W, g);
+        }
       } else if (NG > 1) {
         double b3[3] = {0., 0., 0.};
         CellCache<double> cc;

@@ -2,8 +2,6 @@
 // packing, and the instantiations of the shell-integration kernels.
 #include <cuda_runtime.h>
 
-#include "hxg_adjoint.cuh"
-#include "hxg_adjoint32.cuh"
 #include "hxg_batch.cuh"
 #include "hxg_dispatch.cuh"
 #include "hxg_fp32c.cuh"
@@ -622,37 +620,6 @@ cudaError_t launch_accumulate_transpose(cudaStream_t s, int nside_out,
   const uint64_t n = 12ull * nside_out * nside_out;
   accumulate_transpose_kernel<<<blocks_for(n, 256), 256, 0, s>>>(
       nside_out, nside_shell, g_out, g_shell, scale);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_adjoint(cudaStream_t s, const AdjointLaunch &A,
-                           unsigned blocks, unsigned threads) {
-  const bool ext = A.F.ext != nullptr;
-  const bool fast = fast_models(A.F);
-  if (A.F.ngroups == 0) {
-    if (fast)
-      shell_fp64_adjoint_kernel<0, false, true><<<blocks, threads, 0, s>>>(A);
-    else if (ext)
-      shell_fp64_adjoint_kernel<0, true, false><<<blocks, threads, 0, s>>>(A);
-    else
-      shell_fp64_adjoint_kernel<0, false, false><<<blocks, threads, 0, s>>>(A);
-  } else {
-    if (fast)
-      shell_fp64_adjoint_kernel<1, false, true><<<blocks, threads, 0, s>>>(A);
-    else if (ext)
-      shell_fp64_adjoint_kernel<1, true, false><<<blocks, threads, 0, s>>>(A);
-    else
-      shell_fp64_adjoint_kernel<1, false, false><<<blocks, threads, 0, s>>>(A);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_adjoint32(cudaStream_t s, const AdjointLaunch &A, unsigned blocks,
-                             unsigned threads) {
-  if (A.F.ngroups == 0)
-    shell_fp32c_adjoint_kernel<0><<<blocks, threads, 0, s>>>(A);
-  else
-    shell_fp32c_adjoint_kernel<1><<<blocks, threads, 0, s>>>(A);
   return cudaGetLastError();
 }
 
