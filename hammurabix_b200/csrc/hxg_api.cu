@@ -2576,6 +2576,18 @@ int hxg_read_grid(hxg_handle *h, int field, uint64_t n, const double *pos,
 // ===================================================================
 // batched forward
 // ===================================================================
+using hxg::ShellLaunch;
+
+// A plan launched as a kernel of its own: the launch block, the passes'
+// constants (nf > 1) and its warp tiles.
+struct PlanLaunch {
+  int nf;
+  unsigned long long tiles, work;  // 32-lane tiles; lanes x steps
+  ShellLaunch P;
+  hxg::FreqSet<2> F2;
+  hxg::FreqSet<3> F3;
+};
+
 struct hxg_batch {
   hxg_handle *h = nullptr;
   std::vector<hxg_batch_entry_t> e;
@@ -2595,13 +2607,14 @@ struct hxg_batch {
   std::vector<DevBuf> plans, tiles, merges, mblocks;
   std::vector<int> nplans, nmerge;
   std::vector<unsigned long long> merge_blocks;
+  std::vector<std::vector<PlanLaunch>> direct;  // per level: plans launched one by one
   std::vector<int> group;  // passes fused with entry i (0: inside a group)
   int nzero = 0;
   unsigned long long zero_blocks = 0;
   unsigned level_blocks[3] = {0, 0, 0};
   int graph_kernels = 0;  // kernels one run of the graph launches
   uint64_t layout_gen = 0;  // the handle's layout_gen the graph was made for
-  bool fast = false;        // every entry's models satisfy fast_models
+  bool fast = false;        // every entry's models satisfy fast_models and fast_ok
   cudaGraphExec_t exec = nullptr;
 };
 
@@ -2609,7 +2622,6 @@ namespace {
 
 using hxg::BatchLevel;
 using hxg::MergeJob;
-using hxg::ShellLaunch;
 using hxg::ZeroJob;
 
 bool reads_grid(const hxg_models_t &m, int which) {
@@ -2631,6 +2643,18 @@ int upload_vec(hxg_handle *h, DevBuf &b, const std::vector<T> &v) {
   return HXG_OK;
 }
 
+// A batch level's plans get a kernel each, run side by side in the graph, with
+// the launch block in constant memory and the launch shape of the single
+// pass; the persistent kernel, which reads its plans from global memory at 16
+// warps per SM, is left the FP32C plans of under kSmallTiles warp tiles where
+// a level has more than kManyPlans of them: there the kernels' count (128 run
+// at a time) takes longer than the work.  Measured (ms, persistent / one
+// kernel each): 16 sets x 3 frequencies, Nside 64/128/256 95.8 / 73.1; 24 sets,
+// Nside 16 5.42 / 1.48; 200 sets, Nside 8 2.44 / 1.51; 600 sets, Nside 4/8
+// 2.83 / 3.70.
+constexpr unsigned long long kSmallTiles = 64;
+constexpr size_t kManyPlans = 256;
+
 // Device tables of a batch for one launch shape.
 int batch_tables(hxg_batch *b, int lanes, int grain) {
   hxg_handle *h = b->h;
@@ -2648,6 +2672,16 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
     for (auto &t : t0) t.assign(1, 0ull);
     std::vector<MergeJob> mj;
     std::vector<unsigned long long> m0(1, 0ull);
+    b->direct[s].clear();
+    // pixels of the level, and its plans too small for a kernel of their own
+    uint64_t level_pix = 0;
+    size_t small = 0;
+    for (size_t i = 0; i < b->e.size(); i += (size_t)b->group[i]) {
+      const hxg_obs_t &o = b->e[i].obs;
+      if ((uint32_t)s >= o.total_shell) continue;
+      level_pix += npix_of(o.nside_shell[s]);
+      small += npix_of(o.nside_shell[s]) * (uint64_t)lanes < 32 * kSmallTiles;
+    }
     int tab_st = HXG_OK;
     const auto job = [&](int nmaps, double *const *d, const double *const *src, uint32_t nd,
                          int ns) {
@@ -2674,7 +2708,12 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
       if ((st = build_launch(h, E.models, o, (uint32_t)s, L, step)) != HXG_OK) return st;
       L.mask = nullptr;
       L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) + i : nullptr;
+      // an FP32C batch runs all its plans in one instantiation
+      if (b->fp32 && !b->fast) L.fast_ok = 0;
       int C = std::min(lanes, 32);
+      // the FP64 form cuts a ray's own window, so more lanes cost it little:
+      // enough of them for the level's plans to fill the device
+      if (!b->fp32) C = std::max(C, choose_chunks(h, level_pix, step));
       while (C > 1 && step / (uint64_t)C < 16) C >>= 1;
       L.chunks = C;
       L.log2_chunks = hxg::hpx_ilog2((uint64_t)C);
@@ -2711,6 +2750,8 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
           if (r != HXG_OK) return r;
           F.lambda2[f] = Lf.lambda2;
           F.phase_k[f] = Lf.phase_k;
+          F.quarter_k[f] = Lf.quarter_k;
+          F.quarter_i[f] = Lf.quarter_i;
           F.k_t[f] = Lf.k_t;
           F.k_p[f] = Lf.k_p;
           F.tc_a[f] = Lf.tc_a;
@@ -2721,7 +2762,17 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
         }
         return HXG_OK;
       };
-      if (nf == 1) {
+      const bool alone = !b->fp32 || tiles >= kSmallTiles || small <= kManyPlans;
+      if (alone) {
+        PlanLaunch D{};
+        D.nf = nf;
+        D.tiles = tiles;
+        D.work = tiles * (step / (uint64_t)C);
+        D.P = L;
+        if (nf == 2 && (st = freqs(D.F2)) != HXG_OK) return st;
+        if (nf == 3 && (st = freqs(D.F3)) != HXG_OK) return st;
+        b->direct[s].push_back(D);
+      } else if (nf == 1) {
         P1.push_back(L);
       } else if (nf == 2) {
         hxg::FusedPlan<2> FP;
@@ -2734,7 +2785,7 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
         if ((st = freqs(FP.F)) != HXG_OK) return st;
         P3.push_back(FP);
       }
-      t0[nf - 1].push_back(t0[nf - 1].back() + tiles);
+      if (!alone) t0[nf - 1].push_back(t0[nf - 1].back() + tiles);
       for (int f = 0; f < nf; ++f) {
         const hxg_batch_entry_t &Ef = b->e[i + f];
         const hxg_obs_t &of = Ef.obs;
@@ -2773,6 +2824,57 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
   return HXG_OK;
 }
 
+// The plans of a level with kernels of their own, side by side in the graph
+// that s is capturing: up to kChains chains of kernels (the device runs 128
+// kernels at a time), the heaviest plans first, each to the shortest chain.  A
+// chain's next kernel is captured on s with the chain's last kernel as its
+// dependency.
+cudaError_t launch_direct(hxg_batch *b, std::vector<PlanLaunch> &plans, cudaStream_t s) {
+  constexpr size_t kChains = 128;
+  std::stable_sort(plans.begin(), plans.end(),
+                   [](const PlanLaunch &x, const PlanLaunch &y) { return x.work > y.work; });
+  std::vector<cudaGraphNode_t> deps;
+  const auto here = [&](std::vector<cudaGraphNode_t> &v) {
+    cudaStreamCaptureStatus st;
+    const cudaGraphNode_t *d = nullptr;
+    size_t n = 0;
+    const cudaError_t r = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &d, &n);
+    if (r != cudaSuccess) return r;
+    if (st != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
+    v.assign(d, d + n);
+    return cudaSuccess;
+  };
+  const auto from = [&](std::vector<cudaGraphNode_t> &v) {
+    return cudaStreamUpdateCaptureDependencies(s, v.data(), v.size(),
+                                               cudaStreamSetCaptureDependencies);
+  };
+  cudaError_t e = here(deps);
+  const size_t n = std::min(kChains, plans.size());
+  std::vector<std::vector<cudaGraphNode_t>> tail(n, deps);
+  std::vector<unsigned long long> load(n, 0ull);
+  for (const PlanLaunch &D : plans) {
+    if (e != cudaSuccess) return e;
+    const size_t k = std::min_element(load.begin(), load.end()) - load.begin();
+    load[k] += D.work;
+    if ((e = from(tail[k])) != cudaSuccess) return e;
+    const unsigned threads =
+        !b->fp32 ? HXG_FP64_THREADS : (D.nf == 1 ? HXG_FP32C_THREADS : HXG_FP32C_MULTI_THREADS);
+    const unsigned blocks = (unsigned)((D.tiles * 32 + threads - 1) / threads);
+    if (D.nf == 1)
+      e = hxg::launch_shell(s, b->fp32, D.P, blocks, threads);
+    else
+      e = hxg::launch_shell_multi(s, b->fp32, D.P, D.nf,
+                                  D.nf == 2 ? (const void *)&D.F2 : (const void *)&D.F3, blocks,
+                                  threads);
+    ++b->graph_kernels;
+    if (e == cudaSuccess) e = here(tail[k]);
+  }
+  if (e != cudaSuccess) return e;
+  deps.clear();
+  for (const auto &v : tail) deps.insert(deps.end(), v.begin(), v.end());
+  return from(deps);
+}
+
 void batch_drop_graph(hxg_batch *b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   b->exec = nullptr;
@@ -2803,8 +2905,7 @@ int batch_capture(hxg_batch *b) {
         B.nplans = b->nplans[k];
         B.grain = b->grain;
         B.counter = ctr + k;
-        e = hxg::launch_batch_level(s, b->fp32, b->ngroups, b->ext_any, b->fast, B,
-                                    b->level_blocks[0]);
+        e = hxg::launch_batch_level(s, b->ngroups, b->ext_any, b->fast, B, b->level_blocks[0]);
       } else if (c == 1) {
         hxg::BatchLevelMulti<2> B{static_cast<const hxg::FusedPlan<2> *>(b->plans[k].p), tiles,
                                   b->nplans[k], b->grain, ctr + k};
@@ -2817,6 +2918,8 @@ int batch_capture(hxg_batch *b) {
                                           b->level_blocks[2]);
       }
     }
+    if (e == cudaSuccess && !b->direct[l].empty())
+      e = launch_direct(b, b->direct[l], s);
     if (e != cudaSuccess) break;
     e = hxg::launch_batch_merge(s, static_cast<const MergeJob *>(b->merges[l].p),
                                 static_cast<const unsigned long long *>(b->mblocks[l].p),
@@ -2931,6 +3034,7 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
   b->mblocks.resize(b->levels);
   b->nplans.assign(3 * b->levels, 0);
   b->nmerge.assign(b->levels, 0);
+  b->direct.resize(b->levels);
   b->merge_blocks.assign(b->levels, 0ull);
   const auto bail = [&](int code) {
     batch_free(b);
@@ -2941,12 +3045,12 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
   if ((st = ensure(h, b->counters, 3 * b->levels * sizeof(unsigned long long))) != HXG_OK)
     return bail(st);
   // frequency passes of one parameter set that can share a traversal: up to
-  // three consecutive entries with the same models and geometry (FP32C form,
-  // synchrotron in every pass, no CRE grid)
+  // three consecutive entries with the same models and geometry (synchrotron
+  // in every pass, no CRE grid)
   b->group.assign(b->e.size(), 0);
   for (size_t i = 0; i < b->e.size();) {
     int nf = 1;
-    for (int cand = 3; b->fp32 && cand >= 2 && nf == 1; --cand) {
+    for (int cand = 3; cand >= 2 && nf == 1; --cand) {
       if (i + cand > b->e.size() || b->e[i].models.cre == HXG_CRE_GRID) continue;
       hxg_obs_t o[3];
       bool same = true;
@@ -2985,12 +3089,11 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
     L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) : nullptr;
     b->fast = b->fast && hxg::fast_models(L) && L.fast_ok;
   }
-  int per_sm = 0;
-  cudaError_t ce = hxg::batch_level_occupancy(b->fp32, b->ngroups, b->ext_any, b->fast, &per_sm);
-  if (ce != cudaSuccess) return bail(cuda_fail(h, ce, "occupancy"));
-  b->level_blocks[0] = (unsigned)std::max(1, per_sm) * (unsigned)h->sm_count;
-  for (int nf = 2; nf <= 3 && b->fp32; ++nf) {
-    ce = hxg::batch_multi_occupancy(b->ngroups, b->ext_any, b->fast, nf, &per_sm);
+  cudaError_t ce = cudaSuccess;
+  for (int nf = 1; nf <= 3 && b->fp32; ++nf) {
+    int per_sm = 0;
+    ce = nf == 1 ? hxg::batch_level_occupancy(b->ngroups, b->ext_any, b->fast, &per_sm)
+                 : hxg::batch_multi_occupancy(b->ngroups, b->ext_any, b->fast, nf, &per_sm);
     if (ce != cudaSuccess) return bail(cuda_fail(h, ce, "occupancy"));
     b->level_blocks[nf - 1] = (unsigned)std::max(1, per_sm) * (unsigned)h->sm_count;
   }

@@ -1,14 +1,14 @@
 // hxg_batch.cuh -- batched forward: many independent passes (parameter
 // sets x frequencies) of Integrator::write_grid (integrator.cc:23-134) in
-// one CUDA graph.  Per shell level the graph holds one persistent shell
-// kernel over every entry that has that shell and one kernel that merges
-// the shell maps into each entry's outputs (Hampix::accumulate,
-// hamdis.h:698-721); the outer-shell levels read the inner Faraday depth
-// the earlier levels accumulated (integrator.cc:78-86).
+// one CUDA graph.  Per shell level the graph holds the shell kernels of every
+// parameter set that has that shell, side by side (many small FP32C sets share
+// the persistent kernel below), and one kernel that merges the shell maps into
+// each entry's outputs (Hampix::accumulate, hamdis.h:698-721); the outer-shell
+// levels read the inner Faraday depth the earlier levels accumulated
+// (integrator.cc:78-86).
 #pragma once
 
 #include "hxg_fp32c.cuh"
-#include "hxg_fp64.cuh"
 #include "hxg_integrate.cuh"
 #include "hxg_internal.h"
 
@@ -91,7 +91,7 @@ batch_fp32c_multi_kernel(const BatchLevelMulti<NF> B) {
   batch_multi_body<NG, kExt, NF, kFast>(B);
 }
 
-template <int NG, bool kFp32, bool kExt, bool kFast>
+template <int NG, bool kExt, bool kFast>
 __device__ __forceinline__ void batch_level_body(const BatchLevel &B) {
   const int lane = threadIdx.x & 31;
   const unsigned long long total = B.tile_start[B.nplans];
@@ -112,10 +112,7 @@ __device__ __forceinline__ void batch_level_body(const BatchLevel &B) {
       while (t >= B.tile_start[k + 1]) ++k;
       const ShellLaunch &P = B.plans[k];
       const long long gw = (long long)(t - B.tile_start[k]);
-      if (kFp32)
-        fp32c_tile<NG, kExt, kFast>(P, gw, lane);
-      else
-        fp64_tile<NG, kExt, kFast>(P, gw, lane);
+      fp32c_tile<NG, kExt, kFast>(P, gw, lane);
     }
   }
 }
@@ -125,13 +122,7 @@ __device__ __forceinline__ void batch_level_body(const BatchLevel &B) {
 template <int NG, bool kExt, bool kFast>
 __global__ void __launch_bounds__(256, 2)
 batch_fp32c_kernel(const BatchLevel B) {
-  batch_level_body<NG, true, kExt, kFast>(B);
-}
-
-template <int NG, bool kExt, bool kFast>
-__global__ void __launch_bounds__(256)
-batch_fp64_kernel(const BatchLevel B) {
-  batch_level_body<NG, false, kExt, kFast>(B);
+  batch_level_body<NG, kExt, kFast>(B);
 }
 
 // Map merges of one level: job j adds nmaps shell maps at nside_src into

@@ -76,11 +76,11 @@ cudaError_t launch_adjoint(cudaStream_t s, const AdjointLaunch &A,
 // The FP32C form's adjoint (the grid workloads' models, at most one grid).
 cudaError_t launch_adjoint32(cudaStream_t s, const AdjointLaunch &A, unsigned blocks,
                              unsigned threads);
-// fast: every plan's models satisfy fast_models (the kFast instantiations).
-cudaError_t launch_batch_level(cudaStream_t s, bool fp32, int ngroups, bool ext, bool fast,
+// The persistent FP32C batch kernels.  fast: every plan's models satisfy
+// fast_models (the kFast instantiations).
+cudaError_t launch_batch_level(cudaStream_t s, int ngroups, bool ext, bool fast,
                                const BatchLevel &B, unsigned blocks);
-cudaError_t batch_level_occupancy(bool fp32, int ngroups, bool ext, bool fast,
-                                  int *blocks_per_sm);
+cudaError_t batch_level_occupancy(int ngroups, bool ext, bool fast, int *blocks_per_sm);
 // Fused-frequency plans (nf = 2 or 3): B points to a BatchLevelMulti<nf>.
 cudaError_t launch_batch_level_multi(cudaStream_t s, int ngroups, bool ext, bool fast, int nf,
                                      const void *B, unsigned blocks);

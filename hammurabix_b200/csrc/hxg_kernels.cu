@@ -479,19 +479,15 @@ cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, 
   });
 }
 
-cudaError_t launch_batch_level(cudaStream_t s, bool fp32, int ngroups, bool ext, bool fast,
+cudaError_t launch_batch_level(cudaStream_t s, int ngroups, bool ext, bool fast,
                                const BatchLevel &B, unsigned blocks) {
   return by_shape(ngroups, ext, [&](auto ng, auto ex) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ex)::value;
-    if (fp32 && fast)
+    if (fast)
       batch_fp32c_kernel<NG, false, true><<<blocks, 256, 0, s>>>(B);
-    else if (fp32)
-      batch_fp32c_kernel<NG, E, false><<<blocks, 256, 0, s>>>(B);
-    else if (fast)
-      batch_fp64_kernel<NG, false, true><<<blocks, 256, 0, s>>>(B);
     else
-      batch_fp64_kernel<NG, E, false><<<blocks, 256, 0, s>>>(B);
+      batch_fp32c_kernel<NG, E, false><<<blocks, 256, 0, s>>>(B);
   });
 }
 
@@ -530,20 +526,15 @@ cudaError_t batch_multi_occupancy(int ngroups, bool ext, bool fast, int nf, int 
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, HXG_BATCH_MULTI_THREADS, 0);
 }
 
-cudaError_t batch_level_occupancy(bool fp32, int ngroups, bool ext, bool fast,
-                                  int *blocks_per_sm) {
+cudaError_t batch_level_occupancy(int ngroups, bool ext, bool fast, int *blocks_per_sm) {
   const void *f = nullptr;
   by_shape(ngroups, ext, [&](auto ng, auto ex) {
     constexpr int NG = decltype(ng)::value;
     constexpr bool E = decltype(ex)::value;
-    if (fp32 && fast)
+    if (fast)
       f = (const void *)batch_fp32c_kernel<NG, false, true>;
-    else if (fp32)
-      f = (const void *)batch_fp32c_kernel<NG, E, false>;
-    else if (fast)
-      f = (const void *)batch_fp64_kernel<NG, false, true>;
     else
-      f = (const void *)batch_fp64_kernel<NG, E, false>;
+      f = (const void *)batch_fp32c_kernel<NG, E, false>;
   });
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, 256, 0);
 }

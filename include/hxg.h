@@ -453,17 +453,20 @@ int hxg_adjoint_shard_finish(hxg_handle *h, double *d_grad_params, double *d_gra
  *    analytic parameters may differ); masks are not supported;
  *  - outputs are the caller's device maps (RING), distinct per entry;
  *  - the plan holds per-entry shell temporaries and launch blocks and a
- *    graph with, per shell level, one persistent shell kernel over all
- *    entries (warps take pixel tiles from a work counter) and one kernel
- *    that merges the shell maps into the outputs; an entry's outer shells
- *    read the Faraday depth its inner shells accumulated, as in
+ *    graph with, per shell level, the shell kernels of the parameter sets
+ *    side by side (hundreds of small FP32C sets share one persistent kernel
+ *    instead, whose warps take pixel tiles from a work counter) and one
+ *    kernel that merges the shell maps into the outputs; an entry's outer
+ *    shells read the Faraday depth its inner shells accumulated, as in
  *    write_grid;
- *  - in the FP32C form, up to three consecutive entries with the same
- *    models and geometry and synchrotron output (one parameter set at
- *    several frequencies, as hxg_write_grid_multi takes them; no CRE grid)
- *    share one traversal per shell;
- *  - tune != 0: the launch shapes (lanes per pixel x tiles per fetch) are
- *    timed once in hxg_batch_create and the fastest is kept;
+ *  - up to three consecutive entries with the same models and geometry and
+ *    synchrotron output (one parameter set at several frequencies, as
+ *    hxg_write_grid_multi takes them; no CRE grid) share one traversal per
+ *    shell;
+ *  - tune != 0: the launch shapes (lanes per pixel x tiles per fetch of the
+ *    persistent kernel) are timed once in hxg_batch_create and the fastest is
+ *    kept; the FP64 form takes more lanes where its plans would not fill the
+ *    device;
  *  - hxg_batch_run launches the graph on the handle's stream and does not
  *    synchronise; the entries' host data are not read again;
  *  - grids uploaded to the handle after hxg_batch_create with the same
