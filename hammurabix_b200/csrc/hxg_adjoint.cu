@@ -29,10 +29,15 @@ cudaError_t launch_adjoint(cudaStream_t s, const AdjointLaunch &A,
 
 cudaError_t launch_adjoint32(cudaStream_t s, const AdjointLaunch &A, unsigned blocks,
                              unsigned threads) {
-  if (A.F.ngroups == 0)
-    shell_fp32c_adjoint_kernel<0><<<blocks, threads, 0, s>>>(A);
+  const bool fin = A.F.fast_ok;
+  if (A.F.ngroups == 0 && fin)
+    shell_fp32c_adjoint_kernel<0, true><<<blocks, threads, 0, s>>>(A);
+  else if (A.F.ngroups == 0)
+    shell_fp32c_adjoint_kernel<0, false><<<blocks, threads, 0, s>>>(A);
+  else if (fin)
+    shell_fp32c_adjoint_kernel<1, true><<<blocks, threads, 0, s>>>(A);
   else
-    shell_fp32c_adjoint_kernel<1><<<blocks, threads, 0, s>>>(A);
+    shell_fp32c_adjoint_kernel<1, false><<<blocks, threads, 0, s>>>(A);
   return cudaGetLastError();
 }
 

@@ -3,9 +3,8 @@
 // Given dL/d(shell maps) of one shell, it accumulates dL/d(packed grid
 // records), dL/d(model parameters) and dL/d(inner-shell Faraday-depth map).
 // Per-shell checkpointing: the forward kernel stored, for every (pixel,
-// chunk), the chunk's Faraday depth and its local-frame Q, U sums, plus the
-// pixel's inner-shell Faraday depth.  From those the backward kernel gets,
-// with warp shuffles, the pixel totals Q, U and each chunk's prefix, so a
+// chunk), the Faraday depth before the chunk and Q, U from the chunk on
+// (store_checkpoint), plus the pixel's inner-shell Faraday depth, so a
 // single forward-ordered sweep suffices: the reverse-accumulated phase
 // sensitivity S_i = sum_{k >= i} dL/dchi_k equals
 // 2 (gU (Q - Q_{<i}) - gQ (U - U_{<i})), one running sum since gQ, gU are
@@ -38,13 +37,14 @@ constexpr int kNumParams = 8;
 
 struct AdjointLaunch {
   ShellLaunch F;            // the forward launch of this shell
-  const double *ck;         // [(nest * C + c) * 3]: chunk FD, Q, U (local frame)
+  const double *ck;         // [(nest * C + c) * 3]: store_checkpoint's values
   const double *ck_inner;   // [ring]: inner-shell FD of each pixel
   const double *g[5];       // dL/d(shell maps) (ring): dm, fd, I, Q, U (I,Q,U
                             // already times the temp_convert factor)
   double *grad_rec;         // [N * 4] dL/d(group-0 records), or null
   double *grad_par;         // [kNumParams], or null
   double *g_fdmap;          // [npix(nside_fdmap)] dL/d(accumulated FD map), or null
+  int by_chunk;             // FP32C: a block's lanes take one chunk of 128 pixels
   int want_j0;              // 1 when the CRE normalisation gradient is wanted
 };
 
@@ -111,48 +111,15 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     ring = hpx_nest2ring(h, nest);
     live = (P.mask == nullptr) || (P.mask[ring] != 0);
   }
-  // checkpointed chunk sums; dead lanes contribute zeros to the shuffles
-  double fdc = 0., qc = 0., uc = 0.;
+  // the Faraday depth before this chunk, Q and U from it on
+  double Fc = 0., Qs = 0., Us = 0.;
   if (live) {
     const unsigned long long ci = nest * (unsigned long long)C + c;
-    fdc = A.ck[3 * ci];
-    qc = A.ck[3 * ci + 1];
-    uc = A.ck[3 * ci + 2];
+    Fc = A.ck[3 * ci];
+    Qs = A.ck[3 * ci + 1];
+    Us = A.ck[3 * ci + 2];
   }
   const double l2 = P.lambda2;
-  // exclusive Faraday-depth prefix F_c of the chunks before this one
-  double incl = fdc;
-  for (int o = 1; o < C; o <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, incl, o * S);
-    if (c >= o) incl += v;
-  }
-  double Fc = __shfl_up_sync(0xffffffffu, incl, S);
-  if (c == 0) Fc = 0.;
-  // chunk Q, U in the pixel's (global) phase frame
-  double qg = qc, ug = uc;
-  if (P.do_sync && c > 0) {
-    double sr, cr;
-    sincos(2. * l2 * Fc, &sr, &cr);
-    qg = qc * cr - uc * sr;
-    ug = qc * sr + uc * cr;
-  }
-  double qi = qg, ui = ug;
-  for (int o = 1; o < C; o <<= 1) {
-    const double vq = __shfl_up_sync(0xffffffffu, qi, o * S);
-    const double vu = __shfl_up_sync(0xffffffffu, ui, o * S);
-    if (c >= o) {
-      qi += vq;
-      ui += vu;
-    }
-  }
-  const int last = (C - 1) * S + seg;
-  const double Qp = __shfl_sync(0xffffffffu, qi, last);
-  const double Up = __shfl_sync(0xffffffffu, ui, last);
-  double Qrun = qi - qg, Urun = ui - ug;  // Q, U of the chunks before this one
-  if (c == 0) {
-    Qrun = 0.;
-    Urun = 0.;
-  }
   double gp[kNumParams];
 #pragma unroll
   for (int k = 0; k < kNumParams; ++k) gp[k] = 0.;
@@ -168,7 +135,7 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     // dL/d(inner FD) = lambda^2 sum_i dL/dchi_i, scattered through the
     // transpose of the HEALPix interpolation that produced it
     if (c == 0 && A.g_fdmap != nullptr && P.fdmap != nullptr && P.do_sync) {
-      const double g_inner = l2 * 2. * (gU * Qp - gQ * Up);
+      const double g_inner = l2 * 2. * (gU * Qs - gQ * Us);
       const Hpx hf = hpx_make((uint64_t)P.nside_fdmap);
       uint64_t pix[4];
       double w[4];
@@ -195,7 +162,7 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     const double gIk = gI * P.k_t, gQk = gQ * P.k_p, gUk = gU * P.k_p;
     const double K = P.fd_fore * P.delta, gdmd = gdm * P.delta;
     // gfd + lambda^2 S_i, running: S starts at the chunk's own
-    double gtt = fma(2. * l2, gU * (Qp - Qrun) - gQ * (Up - Urun), gfd);
+    double gtt = fma(2. * l2, gU * Qs - gQ * Us, gfd);
     if (!P.do_sync) gtt = gfd;
     const double l2x2 = 2. * l2;
     // Faraday phase in quarter turns: inner + Fc + the running chunk FD (the

@@ -8,10 +8,18 @@
 // sum, the phase) and the reverse phase sensitivity in FP64; the grid
 // interpolation, the synchrotron emissivity, the polarisation angle and the
 // field gradients in FP32.  The structure follows shell_fp64_adjoint_kernel
-// (hxg_adjoint.cuh): the forward stored, per (pixel, chunk), the chunk's FD
-// and local-frame Q, U, and per pixel the inner-shell FD; one forward-ordered
-// sweep per chunk then forms S_i = 2 (gU (Q - Q_{<i}) - gQ (U - U_{<i})), the
-// sensitivity of the loss to the phase of the samples k >= i.
+// (hxg_adjoint.cuh): one forward-ordered sweep per chunk from the forward's
+// checkpoint keeps gFD + lambda^2 S_i, S_i = 2 (gU (Q - Q_{<i}) -
+// gQ (U - U_{<i})) the sensitivity of the loss to the phase of the samples
+// k >= i.
+//
+// The chunks are the forward's, equal parts of the whole ray, and in the outer
+// shells a ray leaves the cuts in the first of them: with a pixel's chunks in
+// one warp, as in the forward, half of the lanes idle there.  So a block can
+// take 128 neighbouring pixels and one chunk of their rays instead (by_chunk).
+// Where rays are cut late or not at all the forward's mapping stays: near the
+// observer neighbouring rays share their cells, and a warp of 32 of them adds
+// into the same addresses.
 //
 // Per sample, with J_t, Q_i, U_i the sample's emissivity terms in output
 // units and B in 2^-20 G:
@@ -28,10 +36,12 @@
 #include "hxg_adjoint.cuh"
 #include "hxg_fp32c.cuh"
 
-// Launch shape of the FP32C adjoint kernel (threads per block, resident
-// blocks per SM its register allocation must allow).  128 x 4 (128
-// registers) ran the config-4 adjoint in 18.1 ms against 19.3 ms at 128 x 3,
-// 24.4 ms at 128 x 2, 20.3 ms at 128 x 5 and 22.6 ms at 128 x 6.
+// Launch shape of the FP32C adjoint kernel (threads per block = pixels per
+// block, resident blocks per SM its register allocation must allow).  128 x 4
+// (128 registers) runs forward, loss and backward on 256^3 grids, Nside
+// 64/128/256, in 19.6 ms against 20.8 ms at 128 x 3 and 21.2 ms at 128 x 5;
+// 25.9 ms with a pixel's chunks in one warp (16 of 32 lanes active in the
+// outer shell).
 #ifndef HXG_ADJ32_THREADS
 #define HXG_ADJ32_THREADS 128
 #endif
@@ -41,46 +51,31 @@
 
 namespace hxg {
 
-// Adds the accumulators of the cell whose corner 000 is record `key` into
-// the FP64 record gradient and clears them.
-__device__ __forceinline__ void flush_cell32(double *grad_rec, unsigned key, unsigned ny,
-                                             unsigned nz, float acc[8][4]) {
-  if (key == kNoCell) return;
-  const unsigned nyz = ny * nz;
-#pragma unroll
-  for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-      for (int dz = 0; dz < 2; ++dz) {
-        const int k = dx * 4 + dy * 2 + dz;
-        double *p = grad_rec + 4 * (size_t)(key + dx * nyz + dy * nz + dz);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (acc[k][q] != 0.f) atomicAdd(p + q, (double)acc[k][q]);
-          acc[k][q] = 0.f;
-        }
-      }
-}
-
 // Parameter-gradient accumulators of the FP32C adjoint, in the form's units
 // (the host converts): 0 sum B.gB over the spiral samples (dL/dln b0),
 // 1 dL/dpitch, 2 dL/dr_s and 3 dL/dh_s of the spiral (per kpc), 4 sum
 // n_e,disk dL/dn_e (dL/dln n0), 5 dL/dr_s and 6 dL/dh_s of the disk (per
 // kpc), 7 sum dL/dJ J (dL/dln j0).
-template <int NG>
+// kFin: finite launch constants (fast_ok; exp_tab).
+template <int NG, bool kFin>
 __global__ void __launch_bounds__(HXG_ADJ32_THREADS, HXG_ADJ32_MIN_BLOCKS)
 shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
   const ShellLaunch &P = A.F;
   const int lane = threadIdx.x & 31;
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int C = P.chunks;
-  const int seg = lane >> P.log2_chunks;
-  const int c = lane & (C - 1);
+  unsigned long long local = (unsigned long long)blockIdx.x * HXG_ADJ32_THREADS + threadIdx.x;
+  int c = (int)(local & (C - 1));
+  if (A.by_chunk) {
+    // blocks of chunk 0 of every pixel, then of chunk 1, ...
+    const unsigned per_chunk = gridDim.x >> P.log2_chunks;
+    c = (int)(blockIdx.x / per_chunk);
+    local = (unsigned long long)(blockIdx.x % per_chunk) * HXG_ADJ32_THREADS + threadIdx.x;
+  } else {
+    local >>= P.log2_chunks;
+  }
   const Hpx h = hpx_make((uint64_t)P.nside);
   // shard `shard` of `nshards` of the shell (the forward's pixels)
-  const unsigned long long nest =
-      shard_nest(P, (unsigned long long)gw * (32 >> P.log2_chunks) + seg);
+  const unsigned long long nest = shard_nest(P, local);
   const bool valid = nest < h.npix;
   uint64_t ring = 0;
   bool live = false;
@@ -88,48 +83,15 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
     ring = hpx_nest2ring(h, nest);
     live = (P.mask == nullptr) || (P.mask[ring] != 0);
   }
-  // checkpointed chunk sums; dead lanes contribute zeros to the shuffles
-  double fdc = 0., qc = 0., uc = 0.;
+  // the Faraday depth before this chunk, Q and U from it on
+  double Fc = 0., Qs = 0., Us = 0.;
   if (live) {
     const unsigned long long ci = nest * (unsigned long long)C + c;
-    fdc = A.ck[3 * ci];
-    qc = A.ck[3 * ci + 1];
-    uc = A.ck[3 * ci + 2];
+    Fc = A.ck[3 * ci];
+    Qs = A.ck[3 * ci + 1];
+    Us = A.ck[3 * ci + 2];
   }
   const double l2 = P.lambda2;
-  // exclusive Faraday-depth prefix Fc of the chunks before this one
-  double incl = fdc;
-  for (int o = 1; o < C; o <<= 1) {
-    const double v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (c >= o) incl += v;
-  }
-  double Fc = __shfl_up_sync(0xffffffffu, incl, 1);
-  if (c == 0) Fc = 0.;
-  // chunk Q, U in the pixel's (global) phase frame, their prefix and totals
-  double qg = qc, ug = uc;
-  if (P.do_sync && c > 0) {
-    double sr, cr;
-    sincos(2. * l2 * Fc, &sr, &cr);
-    qg = qc * cr - uc * sr;
-    ug = qc * sr + uc * cr;
-  }
-  double qi = qg, ui = ug;
-  for (int o = 1; o < C; o <<= 1) {
-    const double vq = __shfl_up_sync(0xffffffffu, qi, o);
-    const double vu = __shfl_up_sync(0xffffffffu, ui, o);
-    if (c >= o) {
-      qi += vq;
-      ui += vu;
-    }
-  }
-  const int last = (seg << P.log2_chunks) + C - 1;
-  const double Qp = __shfl_sync(0xffffffffu, qi, last);
-  const double Up = __shfl_sync(0xffffffffu, ui, last);
-  double Qrun = qi - qg, Urun = ui - ug;  // Q, U of the chunks before this one
-  if (c == 0) {
-    Qrun = 0.;
-    Urun = 0.;
-  }
   double gp[kNumParams];
 #pragma unroll
   for (int k = 0; k < kNumParams; ++k) gp[k] = 0.;
@@ -145,7 +107,7 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
     // dL/d(inner FD) = lambda^2 sum_i dL/dchi_i, scattered through the
     // transpose of the HEALPix interpolation that produced it
     if (c == 0 && A.g_fdmap != nullptr && P.fdmap != nullptr && P.do_sync) {
-      const double g_inner = l2 * 2. * (gU * Qp - gQ * Up);
+      const double g_inner = l2 * 2. * (gU * Qs - gQ * Us);
       const Hpx hf = hpx_make((uint64_t)P.nside_fdmap);
       uint64_t pix[4];
       double w[4];
@@ -171,6 +133,11 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
     const float spf = F.sp_sinf_s, cpf = F.sp_cosf_s;
     const float pe = F.pe;
     const bool pe2 = P.em_const && P.em_pe == 2.;
+    // dL/d(the sample's weights): the launch scales folded in
+    const double gIk = gI * P.k_t, gQk = gQ * P.k_p, gUk = gU * P.k_p;
+    // gfd + lambda^2 S_i, running: S starts at the chunk's own
+    double gtt = P.do_sync ? fma(2. * l2, gU * Qs - gQ * Us, gfd) : gfd;
+    const double l2x2 = 2. * l2;
     // Faraday phase in turns of the pixel frame: inner + Fc + the running
     // chunk FD (the sample's own term included), rounded as in fp32c_tile
     const double rev0 = l2 * (inner + Fc) * (1. / cgs::pi) + (1572864.0 + 0x1p-24);
@@ -218,20 +185,21 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
       bool in_b = false;
       if (fast_b || fast_t) {
         const double rc2 = fma(px, px, py * py);
-        const double rc2m = fmax(rc2, 1e-300);
+        const double rc2m =
+            __hiloint2double(max(__double2hiint(rc2), 0x01A56E1F), __double2loint(rc2));
         const double y = rsqrt_fd(rc2m);
         r = rc2m * y;
         rcf = float(r);
         in_b = fast_b && !(rc2 > rc2_hi || rc2 < rc2_lo);
         if (in_b) {
           const double ay =
-              exp_tab(fma(-r, F.sp_irs, fma(-fabs(pz), F.sp_ihs, F.sp_crs_l))) * y;
+              exp_tab<kFin>(fma(-r, F.sp_irs, fma(-fabs(pz), F.sp_ihs, F.sp_crs_l))) * y;
           bp_d = ay * fma(K1, d, K0);
           const float ayf = float(ay);
           bxr = ayf * (spf * xf - cpf * yf);
           byr = ayf * (spf * yf + cpf * xf);
         }
-        if (fast_t) te_d = exp_tab(fma(-r, F.ex_irn, fma(-fabs(pz), F.ex_ihn, F.ex_ln0)));
+        if (fast_t) te_d = exp_tab<kFin>(fma(-r, F.ex_irn, fma(-fabs(pz), F.ex_ihn, F.ex_ln0)));
       }
       float bg[4] = {0.f, 0.f, 0.f, 0.f};
       unsigned key = kNoCell;
@@ -263,7 +231,7 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
       double g_bpar = 0.;
       float gbx = 0.f, gby = 0.f, gbz = 0.f;
       if (P.do_fd || P.do_sync) {
-        double gtt = gfd;  // dL/d(sample FD term)
+        const double gk = gtt * P.fd_fore;  // dL/d(sample FD term), S_i with its own phase
         if (P.do_sync) {
           const float bx = bxr + bg[0], by = byr + bg[1], bz = bg[2];
           const float xv = -(epx * bx + epy * by);
@@ -288,26 +256,22 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
           const float ang = (__int_as_float(0x4B400000 + q) - 12582912.0f) * 7.490140565847857e-07f;
           float sf, cf;
           __sincosf(ang, &sf, &cf);
-          const double Qi = P.k_p * (double)fmaf(wpc, cf, -wps * sf);
-          const double Ui = P.k_p * (double)fmaf(wpc, sf, wps * cf);
-          const double Ji = P.k_t * (double)wt;
-          // S_i counts the sample's own phase (k >= i): Q_{<i} before it
-          const double Si = 2. * (gU * (Qp - Qrun) - gQ * (Up - Urun));
-          Qrun += Qi;
-          Urun += Ui;
-          gtt = fma(l2, Si, gtt);
-          const double ej = fma(gI, Ji, fma(gQ, Qi, gU * Ui));
+          const double qi = (double)fmaf(wpc, cf, -wps * sf);
+          const double ui = (double)fmaf(wpc, sf, wps * cf);
+          const double dG = fma(gUk, qi, -(gQk * ui));
+          gtt = fma(-l2x2, dG, gtt);
+          const double ej = fma(gIk, (double)wt, fma(gQk, qi, gUk * ui));
           if (A.want_j0) gp[7] += ej;
           // |B_perp|^pe: e_i pe / |B_perp|^2 B_perp with B_perp =
           // -(xv e_phi + yv e_theta); the angle ipa = atan2(yv, xv)
           const float kb = rr > 0.f ? float(ej) * pe / rr : 0.f;
-          const float ki = rr > 0.f ? float(2. * (gU * Qi - gQ * Ui)) / rr : 0.f;
+          const float ki = rr > 0.f ? float(2. * dG) / rr : 0.f;
           gbx = -kb * fmaf(xv, epx, yv * etx) + ki * fmaf(-xv, etx, yv * epx);
           gby = -kb * fmaf(xv, epy, yv * ety) + ki * fmaf(-xv, ety, yv * epy);
           gbz = -kb * (yv * etz) - ki * (xv * etz);
         }
-        g_te = fma(gtt * bpar, P.fd_fore, g_te);
-        g_bpar = gtt * te * P.fd_fore;
+        g_te = fma(gk, bpar, g_te);
+        g_bpar = gk * te;
       }
       if (!(te_raw > 0.)) g_te = 0.;
       gbx += float(g_bpar * ux);
@@ -332,7 +296,7 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
       if (NG == 1 && key != kNoCell && A.grad_rec != nullptr) {
         const DevGridGroup &G = P.groups[0];
         if (key != acc_key) {
-          flush_cell32(A.grad_rec, acc_key, (unsigned)G.ny, (unsigned)G.nz, acc);
+          flush_cell(A.grad_rec, acc_key, (unsigned)G.ny, (unsigned)G.nz, acc);
           acc_key = key;
         }
         const float wx[2] = {1.f - tx, tx}, wy[2] = {1.f - ty, ty}, wz[2] = {1.f - tz, tz};
@@ -355,7 +319,7 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
       }
     }
     if (NG == 1 && A.grad_rec != nullptr)
-      flush_cell32(A.grad_rec, acc_key, (unsigned)P.groups[0].ny, (unsigned)P.groups[0].nz,
+      flush_cell(A.grad_rec, acc_key, (unsigned)P.groups[0].ny, (unsigned)P.groups[0].nz,
                    acc);
   }
   // parameter gradients: warp reduction, one atomic per warp and slot

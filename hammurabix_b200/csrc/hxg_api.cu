@@ -2123,7 +2123,19 @@ int adjoint_shell(hxg_handle *h, const hxg_obs_t &o, uint32_t s, uint32_t shard,
   if (local == 0) return HXG_OK;
   const uint64_t warps = (local + (32 / C) - 1) / (32 / C);
   const unsigned threads = fp32 ? HXG_ADJ32_THREADS : HXG_ADJ_THREADS;
-  const unsigned blocks = (unsigned)((warps * 32 + threads - 1) / threads);
+  // FP32C: whole blocks of pixels for each chunk in shells whose rays can
+  // leave the cuts in their first 0.4 (hxg_adjoint32.cuh): a lone shell to 30
+  // kpc, cut from 0.33 on, 13.9 against 16.7 ms; one to 20 kpc, cut from 0.5 on,
+  // 4.05 against 3.8 ms, so it keeps the mapping of the forward
+  if (fp32 && C > 1) {
+    double mid = F.d_start + 0.4 * F.delta * (double)F.step, r2 = 0.;
+    for (int k = 0; k < 3; ++k) r2 += F.obs[k] * F.obs[k];
+    const double reach = std::min(F.gc_r_max - std::sqrt(r2),
+                                  std::min(F.gc_z_max - F.obs[2], F.obs[2] - F.gc_z_min));
+    A.by_chunk = reach < mid;
+  }
+  const unsigned blocks = A.by_chunk ? (unsigned)((local + threads - 1) / threads * C)
+                                     : (unsigned)((warps * 32 + threads - 1) / threads);
   HXG_CK(fp32 ? launch_adjoint32(h->stream, A, blocks, threads)
               : launch_adjoint(h->stream, A, blocks, threads));
   ++h->launch_count;

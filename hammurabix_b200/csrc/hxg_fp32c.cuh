@@ -555,14 +555,7 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
       su[f] = ku[f].value() * Fq.k_p[f];
     }
   }
-  // adjoint checkpoint (one pass): the chunk's FD and local-frame Q, U
-  // before the chunk combination, in the FP64 form's units
-  if (NF == 1 && P.ck != nullptr && live) {
-    const unsigned long long ci = nest * (unsigned long long)C + c;
-    P.ck[3 * ci] = fd;
-    P.ck[3 * ci + 1] = sq[0];
-    P.ck[3 * ci + 2] = su[0];
-  }
+  if (NF == 1 && P.ck != nullptr) store_checkpoint(P, live, nest, c, 1, fd, sq[0], su[0]);
   combine_chunks_nf<NF>(P, Fq, c, dm, fd, si, sq, su);
   if (live && c == 0) {
     if (P.do_dm) P.out[0][ring] = dm;

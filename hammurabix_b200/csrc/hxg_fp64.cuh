@@ -205,7 +205,6 @@ __device__ __forceinline__ double bperp_pow64(const ShellLaunch &P, double b2) {
 template <int NG, bool kExt, int NF, bool kFast>
 __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF> &Fq,
                                           long long gw, int lane) {
-  const int C = P.chunks;
   // the warp's 32/C pixels side by side, chunk after chunk: the lanes of a
   // load's quarter warp are neighbouring rays at the same distance, which
   // share cache lines
@@ -411,14 +410,7 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
       su[f] *= Fq.k_p[f];
     }
   }
-  // adjoint checkpoint (one pass): the chunk's FD and local-frame Q, U
-  // before the chunk combination
-  if (NF == 1 && P.ck != nullptr && live) {
-    const unsigned long long ci = nest * (unsigned long long)C + c;
-    P.ck[3 * ci] = fd;
-    P.ck[3 * ci + 1] = sq[0];
-    P.ck[3 * ci + 2] = su[0];
-  }
+  if (NF == 1 && P.ck != nullptr) store_checkpoint(P, live, nest, c, S, fd, sq[0], su[0]);
   combine_chunks_nf<NF>(P, Fq, c, dm, fd, si, sq, su, S);
   if (live && c == 0) {
     if (P.do_dm) P.out[0][ring] = dm;

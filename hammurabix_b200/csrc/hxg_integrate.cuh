@@ -86,8 +86,8 @@ struct ShellLaunch {
   DevModels models;
   DevGridGroup groups[kMaxGroups];
   int ngroups;
-  // adjoint checkpoint (FP64 form): per (pixel, chunk) the chunk's FD, Q, U
-  // before the chunk combination, per pixel the inner-shell FD; null = off
+  // adjoint checkpoint: per (pixel, chunk) what store_checkpoint writes, per
+  // pixel the inner-shell FD; null = off
   double *ck;
   double *ck_inner;
   FastModels fast;
@@ -327,6 +327,44 @@ __device__ __forceinline__ void combine_chunks_nf(const ShellLaunch &P, const Fr
       su[f] += shfl_xor_d(su[f], o * stride);
     }
   }
+}
+
+// The adjoint's checkpoint of one pass, per (pixel, chunk): the Faraday depth
+// of the chunks before it, and Q, U of it and the chunks after it in the
+// pixel's frame (the chunk sums sq, su are in the chunk's own, which starts
+// without the earlier chunks' rotation).  All 32 lanes participate; lanes that
+// are not live store nothing and hold zeros.
+__device__ __forceinline__ void store_checkpoint(const ShellLaunch &P, bool live,
+                                                 unsigned long long nest, int c, int stride,
+                                                 double fd, double sq, double su) {
+  const int C = P.chunks;
+  double incl = fd;
+  for (int o = 1; o < C; o <<= 1) {
+    const double v = __shfl_up_sync(0xffffffffu, incl, o * stride);
+    if (c >= o) incl += v;
+  }
+  double before = C > 1 ? __shfl_up_sync(0xffffffffu, incl, stride) : 0.;
+  if (c == 0) before = 0.;
+  if (P.do_sync && c > 0) {
+    double sr, cr;
+    sincos(2. * P.lambda2 * before, &sr, &cr);
+    const double q = sq * cr - su * sr;
+    su = sq * sr + su * cr;
+    sq = q;
+  }
+  for (int o = 1; o < C; o <<= 1) {
+    const double vq = __shfl_down_sync(0xffffffffu, sq, o * stride);
+    const double vu = __shfl_down_sync(0xffffffffu, su, o * stride);
+    if (c + o < C) {
+      sq += vq;
+      su += vu;
+    }
+  }
+  if (!live) return;
+  const unsigned long long ci = nest * (unsigned long long)C + c;
+  P.ck[3 * ci] = before;
+  P.ck[3 * ci + 1] = sq;
+  P.ck[3 * ci + 2] = su;
 }
 
 // cos(2*ipa), sin(2*ipa) of the IAU polarisation angle
