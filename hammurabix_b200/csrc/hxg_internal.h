@@ -37,10 +37,12 @@ struct InterpTab {
 };
 cudaError_t launch_interp_table(cudaStream_t s, int nside_dst, int nside_src, uint4 *pix,
                                 double2 *w);
-// dst_k += src_k (interpolated when the Nsides differ, from tab when given)
+// dst_k += src_k (interpolated when the Nsides differ, from tab when given);
+// first: dst_k = src_k
 cudaError_t launch_accumulate(cudaStream_t s, int nside_dst, int nside_src,
                               int nmaps, double *const *dst,
-                              const double *const *src, const InterpTab *tab = nullptr);
+                              const double *const *src, const InterpTab *tab = nullptr,
+                              bool first = false);
 cudaError_t launch_pix2ang(cudaStream_t s, int nside, uint64_t n,
                            double *theta, double *phi);
 cudaError_t launch_interpolate(cudaStream_t s, int nside, const double *map,
