@@ -21,7 +21,7 @@
 //
 // The sample is fp64_tile's, in the frame turned by the ray's azimuth (there
 // u = (st, 0, ct), e_theta = (ct, 0, -st), e_phi = (0, 1, 0)); its reverse
-// adds about 90 FP64 instructions to the forward's 161.  The grid-record
+// adds about 90 FP64 instructions to the forward's 170.  The grid-record
 // gradient of a cell is summed in registers while the ray stays in it and
 // flushed with 32 atomic adds at record offsets (the cell index is the offset
 // of its first corner: no divisions).
@@ -152,7 +152,7 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     const double oX = fma(cp, P.obs[0], sp * P.obs[1]);
     const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
     const double YY = fma(Y, Y, 1e-280);
-    const double csY = F.sp_cos_s * Y, ssY = F.sp_sin_s * Y;
+    const double csY = F.sp_cos * Y, ssY = F.sp_sin * Y;
     const bool fast_b = M.breg == kBregSpiral;
     const bool fast_t = M.tereg == kTeregExpdisk;
     const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
@@ -178,8 +178,8 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     double sfd = 0.;  // running FD of this chunk (FD-sum units)
     int i0, i1;
     chunk_range64(P, u, c, i0, i1);
-    GridRay64 R;
-    if (NG == 1) grid_ray64(P, P.groups[0], u, i0, i1, R);
+    int ga = i1, gb = i1;
+    if (NG == 1) grid_range64(P, P.groups[0], u, i0, i1, ga, gb);
     double x = (double)i0 + 0.5;
 #pragma unroll 1
     for (int i = i0; i < i1; ++i, x += 1.) {
@@ -196,22 +196,23 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
       double g[4] = {0., 0., 0., 0.};
       Cell64 W;
       W.key = kNoCell;
-      if (NG == 1 && (unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) {
-        cell_of64(P.groups[0], R, d, W);
+      if (NG == 1 && (unsigned)(i - ga) < (unsigned)(gb - ga)) {
+        cell_of64(P.groups[0], u, d, W);
         trilinear64(P.groups[0], W, g);
       }
-      const double ir = rsqrt64(r2), r = r2 * ir;
+      double ir;
+      const double r = sqrt64(r2, ir);
       const double az = fabs(z);
       double sX = 0., sY = 0., bX = 0., bY = 0., bz = 0., te_d = 0.;
       if (fast_b && __double_as_longlong(r2) >= __double_as_longlong(F.rc2_lo) &&
           __double_as_longlong(r2) <= __double_as_longlong(F.rc2_hi)) {
-        const double a = exp64<!kFast>(fma(F.sp_rsun - r, F.sp_irs, -(az * F.sp_ihs))) * ir;
-        sX = a * fma(F.sp_sin_s, X, -csY);
-        sY = a * fma(F.sp_cos_s, X, ssY);
+        const double a = F.sp_b0 * (exp64<!kFast>(spiral_arg64(F, r, az)) * ir);
+        sX = a * fma(F.sp_sin, X, -csY);
+        sY = a * fma(F.sp_cos, X, ssY);
       }
       bX = sX;
       bY = sY;
-      if (fast_t) te_d = F.ex_n0 * exp64<!kFast>(-fma(r, F.ex_irn, az * F.ex_ihn));
+      if (fast_t) te_d = F.ex_n0 * exp64<!kFast>(disk_arg64(F, r, az));
       double te = te_d;
       if (slow_b) {
         const V3<double> B = breg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);

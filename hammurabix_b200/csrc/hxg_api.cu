@@ -642,6 +642,12 @@ int choose_chunks(const hxg_handle *h, uint64_t npix, uint64_t step) {
   return c;
 }
 
+// What the double ia = 1/a misses of it; 0 for a zero or infinite a.
+double reciprocal_rest(double a, double ia) {
+  const double r = (double)(1.L / a - ia);
+  return std::isfinite(r) ? r : 0.;
+}
+
 // All launch constants of one shell (integrator.cc:136-228 semantics).
 int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
                  uint32_t s, ShellLaunch &P, uint64_t &step_out) {
@@ -715,11 +721,20 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
       const double e = 0.5 * (idx + 1);
       P.em_pow_kind = (e == -1.) ? 1 : (e == 0. ? 2 : 0);
       P.em_pe = 1. - e;
-      double ae = std::pow(a_s, e);
-      // bperp_pow64 takes |B_perp|^2 in 2^-40 G^2
-      if (!fp32 && P.em_pe != 2.) ae *= std::pow(2., -20. * P.em_pe);
+      const double ae = std::pow(a_s, e);
       P.k_t = kbase / P.em_den_t * ae * P.em_gt * delta * P.i2bt;
       P.k_p = kbase / P.em_den_p * ae * P.em_gp * delta * P.i2bt;
+      if (!fp32) {
+        // one rounding: these scale a whole map, where the reference rounds
+        // the same factors sample by sample
+        using ld = long double;
+        ld k = (ld)P.em_n0u * 1.73205081 * P.em_qe3 * delta * P.i2bt *
+               std::pow((ld)P.em_anum / (ld)P.em_3qe, (ld)e);
+        // bperp_pow64 takes |B_perp|^2 in 2^-40 G^2
+        if (P.em_pe != 2.) k *= std::pow((ld)2., (ld)(-20. * P.em_pe));
+        P.k_t = (double)(k * P.em_gt / P.em_den_t);
+        P.k_p = (double)(k * P.em_gp / P.em_den_p);
+      }
     } else {
       P.k_t = kbase / (4. * cgs::pi * mec2) * delta * P.i2bt;
       P.k_p = kbase / P.em_den_p * delta * P.i2bt;
@@ -771,8 +786,10 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     const long double quarter = 4.L * P.lambda2 / 3.14159265358979323846264338327950288L;
     P.quarter_i = (double)quarter;
     P.quarter_k = (double)(quarter * fdfore * delta);
-    F.sp_sin_s = D.sp_b0 * D.sp_sin;
-    F.sp_cos_s = D.sp_b0 * D.sp_cos;
+    F.sp_irs_l = reciprocal_rest(D.sp_rs, F.sp_irs);
+    F.sp_ihs_l = reciprocal_rest(D.sp_hs, F.sp_ihs);
+    F.ex_irn_l = reciprocal_rest(D.tex_rs, F.ex_irn);
+    F.ex_ihn_l = reciprocal_rest(D.tex_hs, F.ex_ihn);
     F.cre64_R0 = D.cre_R0;
     F.cre64_ir0 = 1. / D.cre_r0;
     F.cre64_2iz0 = 2. / std::fabs(D.cre_z0);
@@ -803,9 +820,15 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
     D.lo[0] = G.desc.x_min * L;
     D.lo[1] = G.desc.y_min * L;
     D.lo[2] = G.desc.z_min * L;
+    const double lo[3] = {D.lo[0], D.lo[1], D.lo[2]};
     D.scale[0] = (double)(G.desc.nx - 1) / ((G.desc.x_max - G.desc.x_min) * L);
     D.scale[1] = (double)(G.desc.ny - 1) / ((G.desc.y_max - G.desc.y_min) * L);
     D.scale[2] = (double)(G.desc.nz - 1) / ((G.desc.z_max - G.desc.z_min) * L);
+    for (int k = 0; k < 3; ++k) {
+      const long double ol = (long double)P.obs[k] - lo[k];
+      D.ol[k] = (double)ol;
+      D.gl[k] = (double)((ol - D.ol[k]) * D.scale[k]);
+    }
   }
   return HXG_OK;
 }

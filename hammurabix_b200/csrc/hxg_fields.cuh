@@ -230,6 +230,7 @@ struct DevGridGroup {
   double lo[3];     // box minimum (working length units)
   double scale[3];  // (n - 1) / (max - min)
   double gmax[3];   // n - 1: the grid coordinate of the upper box face
+  double ol[3], gl[3];  // observer - lo, and its rounding in grid coordinates
 };
 
 template <typename T>

@@ -16,7 +16,11 @@
 //     not the whole ray, is cut into the chunks of a pixel's lanes;
 //   - divisions by model parameters are products with their reciprocals, the
 //     remaining functions come from hxg_math64.cuh, two exponentials of one
-//     product are one, and launch constants multiply the sums once;
+//     product are one, and launch constants multiply the sums once; constants
+//     whose rounding would act on every sample alike (reciprocals, the
+//     observer's grid coordinates, the emissivity scale) are kept in two parts
+//     or made in extended precision, so that the maps are as near to the exact
+//     ones as with the reference's operations, which round sample by sample;
 //   - |B_perp|^2 of CRE index 3 needs neither root nor power, and the angle's
 //     cos 2ipa, sin 2ipa never divide by |B_perp|^2;
 //   - up to three frequency passes of one geometry share the traversal: a
@@ -26,8 +30,8 @@
 // 34.4 ms before these, 19.4 ms with the sample arithmetic, 14.4 ms with the
 // window cut into chunks and the coefficients as constant operands (30 of 32
 // lanes active against 20), 13.1 ms with quarter warps of neighbouring rays at
-// 128 x 5, 11.6 ms with 32-byte record loads.  A sample is 161 FP64
-// instructions, 80 clocks of an SM's FP64 pipes, and about as many of its L1
+// 128 x 5, 11.6 ms with 32-byte record loads.  A sample is 170 FP64
+// instructions, 85 clocks of an SM's FP64 pipes, and about as many of its L1
 // data stage (8 records of 32 bytes for each of 32 lanes); the two together
 // bound the loop, each about 60 % busy.
 #pragma once
@@ -79,34 +83,39 @@ __device__ __forceinline__ void chunk_range64(const ShellLaunch &P, const double
   i1 = (int)(lo + ((n * (c + 1)) >> P.log2_chunks));
 }
 
-// The ray's coordinates in a grid group, g(d) = g0 + gv d per axis, and the
-// samples [ga, gb) of [i0, i1) that lie inside its box (0 < g < n - 1 on
-// every axis, breg.cc:34-54): the slab intersections, widened by two samples
-// and trimmed with the test itself (the rounded g(d) is monotone in d).
-struct GridRay64 {
+// Grid coordinate k of the ray at distance d: (observer - lo + u d) scale, the
+// rounding of observer - lo, which would move every sample of every ray the
+// same way, added back.
+__device__ __forceinline__ double grid_at64(const DevGridGroup &G, double u, int k, double d) {
+  return fma(fma(u, d, G.ol[k]), G.scale[k], G.gl[k]);
+}
+
+// The samples [ga, gb) of [i0, i1) of a ray that lie inside a grid group's box
+// (0 < g < n - 1 on every axis, breg.cc:34-54): the slab intersections, widened
+// by two samples and trimmed with the test itself (the rounded grid coordinate
+// is monotone in d).
+__device__ __forceinline__ void grid_range64(const ShellLaunch &P, const DevGridGroup &G,
+                                             const double u[3], int i0, int i1, int &ga,
+                                             int &gb) {
   double g0[3], gv[3];
-  int ga, gb;
-};
-__device__ __forceinline__ void grid_ray64(const ShellLaunch &P, const DevGridGroup &G,
-                                           const double u[3], int i0, int i1, GridRay64 &R) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    R.g0[k] = (P.obs[k] - G.lo[k]) * G.scale[k];
-    R.gv[k] = u[k] * G.scale[k];
+    g0[k] = G.ol[k] * G.scale[k];
+    gv[k] = u[k] * G.scale[k];
   }
-  grid_window(P, G, R.g0, R.gv, i0, i1, R.ga, R.gb);
+  grid_window(P, G, g0, gv, i0, i1, ga, gb);
   const auto in = [&](int i) {
     const double d = fma((double)i + 0.5, P.delta, P.d_start);
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double g = fma(R.gv[k], d, R.g0[k]);
+      const double g = grid_at64(G, u[k], k, d);
       ok = ok && g > 0. && g < G.gmax[k];
     }
     return ok;
   };
-  while (R.ga < R.gb && !in(R.ga)) ++R.ga;
-  while (R.gb > R.ga && !in(R.gb - 1)) --R.gb;
+  while (ga < gb && !in(ga)) ++ga;
+  while (gb > ga && !in(gb - 1)) --gb;
 }
 
 // Cell and fraction of a grid coordinate 0 < g < 2^31: adding 2^52 rounded
@@ -130,13 +139,13 @@ struct Cell64 {
   unsigned key;
   double w4[4], ez, fz;
 };
-__device__ __forceinline__ void cell_of64(const DevGridGroup &G, const GridRay64 &R, double d,
+__device__ __forceinline__ void cell_of64(const DevGridGroup &G, const double u[3], double d,
                                           Cell64 &W) {
   int cx, cy, cz;
   double fx, fy;
-  cell64(fma(R.gv[0], d, R.g0[0]), cx, fx);
-  cell64(fma(R.gv[1], d, R.g0[1]), cy, fy);
-  cell64(fma(R.gv[2], d, R.g0[2]), cz, W.fz);
+  cell64(grid_at64(G, u[0], 0, d), cx, fx);
+  cell64(grid_at64(G, u[1], 1, d), cy, fy);
+  cell64(grid_at64(G, u[2], 2, d), cz, W.fz);
   W.key = ((unsigned)cx * (unsigned)G.ny + (unsigned)cy) * (unsigned)G.nz + (unsigned)cz;
   const double ex = 1. - fx, ey = 1. - fy;
   W.ez = 1. - W.fz;
@@ -175,6 +184,18 @@ __device__ __forceinline__ void trilinear64(const DevGridGroup &G, const Cell64 
     out[2] = fma(wb, b1.x, out[2]);
     out[3] = fma(wb, b1.y, out[3]);
   }
+}
+
+// (rs - r) / r_s - |z| / h_s of the spiral, -(r / r_s + |z| / h_s) of the disk,
+// with reciprocals in two parts.
+__device__ __forceinline__ double spiral_arg64(const FastModels &F, double r, double az) {
+  const double s = F.sp_rsun - r;
+  const double t = fma(az, F.sp_ihs_l, fma(-s, F.sp_irs_l, az * F.sp_ihs));
+  return fma(s, F.sp_irs, -t);
+}
+__device__ __forceinline__ double disk_arg64(const FastModels &F, double r, double az) {
+  const double t = fma(az, F.ex_ihn_l, fma(r, F.ex_irn_l, az * F.ex_ihn));
+  return -fma(r, F.ex_irn, t);
 }
 
 // CRE_ana spatial profile exp((R0 - r)/r0) sech^2(z/z0) (cre_ana.cc:11-63):
@@ -244,7 +265,7 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
     const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
     // r^2 along the ray is X^2 + YY; never 0, so that 1/r is finite
     const double YY = fma(Y, Y, 1e-280);
-    const double csY = F.sp_cos_s * Y, ssY = F.sp_sin_s * Y;
+    const double csY = F.sp_cos * Y, ssY = F.sp_sin * Y;
     const bool fast_b = M.breg == kBregSpiral;
     const bool fast_t = M.tereg == kTeregExpdisk;
     const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
@@ -259,8 +280,8 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
     double sdm = 0., sfd = 0., last_index = nan(""), gt = P.em_gt, gp = P.em_gp;
     int i0, i1;
     chunk_range64(P, u, c, i0, i1);
-    GridRay64 R;
-    if (NG == 1) grid_ray64(P, P.groups[0], u, i0, i1, R);
+    int ga = i1, gb = i1;
+    if (NG == 1) grid_range64(P, P.groups[0], u, i0, i1, ga, gb);
     double x = (double)i0 + 0.5;
 #pragma unroll 1
     for (int i = i0; i < i1; ++i, x += 1.) {
@@ -278,9 +299,9 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
       // the grid first: its loads return while the models are evaluated
       double g[4] = {0., 0., 0., 0.};
       if (NG == 1) {
-        if ((unsigned)(i - R.ga) < (unsigned)(R.gb - R.ga)) {
+        if ((unsigned)(i - ga) < (unsigned)(gb - ga)) {
           Cell64 W;
-          cell_of64(P.groups[0], R, d, W);
+          cell_of64(P.groups[0], u, d, W);
           trilinear64(P.groups[0], W, g);
         }
       } else if (NG > 1) {
@@ -293,17 +314,18 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
         g[1] = b3[1];
         g[2] = b3[2];
       }
-      const double ir = rsqrt64(r2), r = r2 * ir;
+      double ir;
+      const double r = sqrt64(r2, ir);
       const double az = fabs(z);
       double bX = 0., bY = 0., bz = 0., te = 0.;
       // positive doubles compare like integers, off the FP64 pipe
       if (fast_b && __double_as_longlong(r2) >= __double_as_longlong(F.rc2_lo) &&
           __double_as_longlong(r2) <= __double_as_longlong(F.rc2_hi)) {
-        const double a = exp64<!kFast>(fma(F.sp_rsun - r, F.sp_irs, -(az * F.sp_ihs))) * ir;
-        bX = a * fma(F.sp_sin_s, X, -csY);
-        bY = a * fma(F.sp_cos_s, X, ssY);
+        const double a = F.sp_b0 * (exp64<!kFast>(spiral_arg64(F, r, az)) * ir);
+        bX = a * fma(F.sp_sin, X, -csY);
+        bY = a * fma(F.sp_cos, X, ssY);
       }
-      if (fast_t) te = F.ex_n0 * exp64<!kFast>(-fma(r, F.ex_irn, az * F.ex_ihn));
+      if (fast_t) te = F.ex_n0 * exp64<!kFast>(disk_arg64(F, r, az));
       if (slow_b) {
         const V3<double> B = breg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
         bX = fma(cp, B.x, sp * B.y);

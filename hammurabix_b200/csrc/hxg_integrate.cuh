@@ -31,8 +31,10 @@ struct FastModels {
   // r_sun/r_s + ln|b0| and ln n0, the sign of b0 into sp_*_s
   double sp_crs_l, ex_ln0;
   double sp_sin_s, sp_cos_s;             // sign(b0) sin, sign(b0) cos
-                                         // (FP64 form: b0 sin, b0 cos)
   double sp_rsun;                        // r_sun
+  // FP64 form: the rounding of sp_irs, sp_ihs, ex_irn, ex_ihn, which would
+  // move every sample's exponent the same way
+  double sp_irs_l, sp_ihs_l, ex_irn_l, ex_ihn_l;
   double cre64_R0, cre64_ir0, cre64_2iz0;  // CRE_ana: R0, 1/r0, 2/|z0|
   float sp_sinf_s, sp_cosf_s;            // the same in FP32
   // launch constants in the types the sample loop uses, so that the loop

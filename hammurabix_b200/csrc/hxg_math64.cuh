@@ -87,6 +87,14 @@ __device__ __forceinline__ double rsqrt64(double t) {
   return fma(y * e, fma(e, kC64.r3, 0.5), y);
 }
 
+// sqrt(t) and ir = 1/sqrt(t) for normal t > 0; one Newton step on the root, so
+// that it is good to half an ulp and a little.
+__device__ __forceinline__ double sqrt64(double t, double &ir) {
+  ir = rsqrt64(t);
+  const double r = t * ir;
+  return fma(fma(-r, r, t), 0.5 * ir, r);
+}
+
 // 1/d for normal d to about one ulp: the hardware estimate and one
 // third-order step.
 __device__ __forceinline__ double rcp64(double d) {
