@@ -53,6 +53,9 @@ struct Group {
 
 }  // namespace
 
+// Bytes of output maps up to which a host-buffer call copies them in one piece.
+constexpr size_t kLanding = 1u << 20;
+
 struct hxg_handle {
   int device = 0;
   int precision = HXG_FP64;
@@ -85,7 +88,9 @@ struct hxg_handle {
   std::map<uint64_t, DevBuf> interp;
   size_t interp_bytes = 0;
   size_t interp_limit = 8ull << 30;
-  DevBuf out[5];
+  DevBuf out;  // device maps of the host-buffer calls
+  // pinned landing zone of small host-buffer calls (kLanding bytes, on first use)
+  char *landing = nullptr;
   bool timing = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
   std::vector<int64_t> event_samples;
@@ -1020,8 +1025,8 @@ int hxg_destroy(hxg_handle *h) {
   if (h->up_stream) cudaStreamDestroy(h->up_stream);
   if (h->shell_all.p) cudaFree(h->shell_all.p);
   for (auto &kv : h->interp) cudaFree(kv.second.p);
-  for (auto &b : h->out)
-    if (b.p) cudaFree(b.p);
+  if (h->out.p) cudaFree(h->out.p);
+  if (h->landing) cudaFreeHost(h->landing);
   for (auto &b : h->ck)
     if (b.p) cudaFree(b.p);
   for (auto &b : h->ck_inner)
@@ -1944,17 +1949,33 @@ int hxg_write_grid_multi_host(hxg_handle *h, int npass, const hxg_obs_t *obs,
         return fail(h, HXG_ERR_INVALID, "pass %d: output %d requested but NULL", k, j);
       total += count(obs[k], j);
     }
-  int st = ensure(h, h->out[0], std::max<size_t>(total, 1) * sizeof(double));
+  int st = ensure(h, h->out, std::max<size_t>(total, 1) * sizeof(double));
   if (st != HXG_OK) return st;
   std::vector<double *> dev(5 * npass, nullptr);
-  double *base = static_cast<double *>(h->out[0].p);
-  for (int k = 0, off = 0; k < npass; ++k)
+  double *base = static_cast<double *>(h->out.p);
+  size_t off = 0;
+  for (int k = 0; k < npass; ++k)
     for (int j = 0; j < 5; ++j)
       if (const size_t c = count(obs[k], j)) {
         dev[5 * k + j] = base + off;
-        off += (int)c;
+        off += c;
       }
   if ((st = hxg_write_grid_multi(h, npass, obs, dev.data())) != HXG_OK) return st;
+  // Small maps cross in one copy into pinned memory: a copy into the caller's
+  // pageable array takes 10 us and more each and waits for the one before it.
+  const size_t bytes = total * sizeof(double);
+  if (bytes <= kLanding &&
+      (h->landing || cudaMallocHost((void **)&h->landing, kLanding) == cudaSuccess)) {
+    HXG_CK(cudaMemcpyAsync(h->landing, base, bytes, cudaMemcpyDeviceToHost, h->stream));
+    HXG_CK(cudaStreamSynchronize(h->stream));
+    for (int k = 0; k < npass; ++k)
+      for (int j = 0; j < 5; ++j)
+        if (const size_t c = count(obs[k], j))
+          std::memcpy(outs[5 * k + j], h->landing + (dev[5 * k + j] - base) * sizeof(double),
+                      c * sizeof(double));
+    return HXG_OK;
+  }
+  (void)cudaGetLastError();  // no pinned memory to be had: copy directly
   for (int k = 0; k < npass; ++k)
     for (int j = 0; j < 5; ++j)
       if (const size_t c = count(obs[k], j))
@@ -2335,24 +2356,8 @@ int hxg_write_grid(hxg_handle *h, const hxg_obs_t *o, double *dm, double *fd,
   if (st != HXG_OK) return st;
   if ((o->do_dm && !dm) || (o->do_fd && !fd) || (o->do_sync && (!is || !qs || !us)))
     return fail(h, HXG_ERR_INVALID, "an output requested by obs is NULL");
-  const size_t b_dm = o->do_dm ? npix_of(o->nside_dm) * 8 : 8;
-  const size_t b_fd = o->do_fd ? npix_of(o->nside_fd) * 8 : 8;
-  const size_t b_sy = o->do_sync ? npix_of(o->nside_sync) * 8 : 8;
-  const size_t bytes[5] = {b_dm, b_fd, b_sy, b_sy, b_sy};
-  for (int k = 0; k < 5; ++k)
-    if ((st = ensure(h, h->out[k], bytes[k])) != HXG_OK) return st;
-  double *d[5];
-  for (int k = 0; k < 5; ++k) d[k] = static_cast<double *>(h->out[k].p);
-  st = hxg_write_grid_device(h, o, d[0], d[1], d[2], d[3], d[4]);
-  if (st != HXG_OK) return st;
-  double *host[5] = {dm, fd, is, qs, us};
-  const bool want[5] = {o->do_dm != 0, o->do_fd != 0, o->do_sync != 0,
-                        o->do_sync != 0, o->do_sync != 0};
-  for (int k = 0; k < 5; ++k)
-    if (want[k])
-      HXG_CK(cudaMemcpyAsync(host[k], d[k], bytes[k], cudaMemcpyDeviceToHost, h->stream));
-  HXG_CK(cudaStreamSynchronize(h->stream));
-  return HXG_OK;
+  double *const outs[5] = {dm, fd, is, qs, us};
+  return hxg_write_grid_multi_host(h, 1, o, outs);
 }
 
 int hxg_sync(hxg_handle *h) {
