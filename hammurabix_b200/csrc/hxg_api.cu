@@ -535,7 +535,14 @@ void ext_models(const hxg_models_t &m, double L, double Bu, ExtModels &x) {
     F.cot_inc = 1 / std::tan(cgs::pi / 180. * (90 - inc));
     F.sin_inc = std::sin(cgs::pi / 180. * inc);
     F.cos_inc = std::cos(cgs::pi / 180. * inc);
-    F.tan_x = std::tan(m.jf12.Xtheta);
+    F.cot_x = 1. / std::tan(m.jf12.Xtheta);
+    F.cos_x = std::cos(m.jf12.Xtheta);
+    F.sin_x = std::sin(m.jf12.Xtheta);
+    F.turn = std::exp(-2. * cgs::pi * F.cot_inc);
+    F.i2w_disk = 2. / F.p.w_disk;
+    F.i2wh = 2. / F.p.wh;
+    F.iz0 = 1. / F.p.z0;
+    F.ir0_X = 1. / F.p.r0_X;
     F.r_max = 20 * cgs::kpc * L;
     F.rho_gc = 1. * cgs::kpc * L;
     F.r_min = 5. * cgs::kpc * L;

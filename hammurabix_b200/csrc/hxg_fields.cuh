@@ -167,8 +167,9 @@ __device__ __forceinline__ T tereg_model(const DevModels &m, T x, T y, T z,
 }
 
 // Regular B and n_e including the models of hxg_models_ext.cuh (FP64).
-// kExt = false instantiations compile to breg_model / tereg_model alone.
-template <bool kExt>
+// kExt = false instantiations compile to breg_model / tereg_model alone;
+// kInline: JF12 in line.
+template <bool kExt, bool kInline = false>
 __device__ __forceinline__ V3<double> breg_model_x(const DevModels &m, const ExtModels *ext,
                                                    double x, double y, double z,
                                                    const double p[3]) {
@@ -176,6 +177,8 @@ __device__ __forceinline__ V3<double> breg_model_x(const DevModels &m, const Ext
     double bb[3];
     if (m.breg == kBregJaffe)
       breg_jaffe(ext->jaffe, x, y, z, bb);
+    else if (kInline)
+      jf12_field(ext->jf12, x, y, z, bb);
     else
       breg_jf12(ext->jf12, x, y, z, bb);
     return V3<double>{bb[0], bb[1], bb[2]};

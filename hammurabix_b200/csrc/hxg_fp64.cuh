@@ -48,6 +48,11 @@
 #ifndef HXG_FP64_MIN_BLOCKS
 #define HXG_FP64_MIN_BLOCKS 5
 #endif
+// With the Jaffe / JF12 / YMW16 models 128 x 4 (128 registers): the masked JF12
+// pass of hxg_models_ext.cuh in 2.03 ms against 2.10 ms at 128 x 5.
+#ifndef HXG_FP64_EXT_MIN_BLOCKS
+#define HXG_FP64_EXT_MIN_BLOCKS 4
+#endif
 // The fused kernels: three passes over Nside 128-1024 on 512^3 grids 91.7 ms
 // (205.3 ms pass by pass; 94.4 at 128 x 4, 95.4 at 128 x 6), two passes over
 // the case above 6.8 ms (7.2, 7.1).
@@ -327,7 +332,7 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
       }
       if (fast_t) te = F.ex_n0 * exp64<!kFast>(disk_arg64(F, r, az));
       if (slow_b) {
-        const V3<double> B = breg_model_x<kExt>(M, P.ext, p3[0], p3[1], p3[2], p3);
+        const V3<double> B = breg_model_x<kExt, true>(M, P.ext, p3[0], p3[1], p3[2], p3);
         bX = fma(cp, B.x, sp * B.y);
         bY = fma(cp, B.y, -(sp * B.x));
         bz = B.z;
@@ -466,7 +471,8 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, long long gw, in
 }
 
 template <int NG, bool kExt, bool kFast>
-__global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MIN_BLOCKS)
+__global__ void __launch_bounds__(HXG_FP64_THREADS,
+                                  kExt ? HXG_FP64_EXT_MIN_BLOCKS : HXG_FP64_MIN_BLOCKS)
 shell_fp64_kernel(const ShellLaunch P) {
   fp64_tile<NG, kExt, kFast>(P, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                              threadIdx.x & 31);
@@ -474,7 +480,8 @@ shell_fp64_kernel(const ShellLaunch P) {
 
 // NF frequency passes in one traversal of the shell.
 template <int NG, bool kExt, int NF, bool kFast>
-__global__ void __launch_bounds__(HXG_FP64_THREADS, HXG_FP64_MULTI_MIN_BLOCKS)
+__global__ void __launch_bounds__(HXG_FP64_THREADS,
+                                  kExt ? HXG_FP64_EXT_MIN_BLOCKS : HXG_FP64_MULTI_MIN_BLOCKS)
 shell_fp64_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
   fp64_tile<NG, kExt, NF, kFast>(P, Fq, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                                  threadIdx.x & 31);
