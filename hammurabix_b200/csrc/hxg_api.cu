@@ -1352,7 +1352,7 @@ int hxg_generate_ternd_dft(hxg_handle *h, const hxg_grid_desc_t *g,
   if (st != HXG_OK) return st;
   Slot &S = h->slots[HXG_FIELD_TERND];
   st = generate_ternd_dft(h->stream, h->rfg, *g, *p, observer, rfg_seed(seed), S.d[0]);
-  h->launch_count += 4;  // fill, two reduction passes, rescale
+  h->launch_count += 7;  // axes, fill, four reductions, rescale
   if (st != HXG_OK) return rfg_result(h, st, "ternd_dft");
   S.present = true;
   h->groups_dirty = true;
@@ -1409,7 +1409,7 @@ int hxg_generate_brnd_es(hxg_handle *h, const hxg_grid_desc_t *g, const hxg_brnd
   Slot &S = h->slots[HXG_FIELD_BRND];
   st = generate_brnd_es(h->stream, h->rfg, *g, *p, M, xb.p, bg, rfg_seed(seed), S.d[0], S.d[1],
                         S.d[2]);
-  h->launch_count += 7;  // fill, two reductions, rescale, project, repack, final
+  h->launch_count += 9;  // axes, fill, four reductions, rescale, project, final
   if (st != HXG_OK) return rfg_result(h, st, "brnd_es");
   S.present = true;
   h->groups_dirty = true;

@@ -60,9 +60,9 @@ __device__ inline void gauss4(uint64_t seed, uint64_t idx, double g[4]) {
   }
 #pragma unroll
   for (int q = 0; q < nb; ++q) {
-    const double r = sqrt(-2. * log(u[2 * q]));
-    double s, c;
-    sincospi(2. * u[2 * q + 1], &s, &c);
+    double ir, s, c;
+    const double r = sqrt64(fmax(-2. * log(u[2 * q]), 1e-280), ir);  // u rounds to 1 at most
+    sincos_quarter(4. * u[2 * q + 1], s, c);
     g[2 * q] = r * c;
     g[2 * q + 1] = r * s;
   }
@@ -76,10 +76,30 @@ __device__ inline double kcomp(int i, int n, double L) {
   return k;
 }
 
+// x^a for normal x > 0 to about one ulp: x = 2^E m with m in [0.7, 1.42), and
+// a E split into an integer and a rest, so that the argument of the one
+// exponential stays below about |a| / 2 and its rounding with it.
+__device__ inline double pow_k(double x, double a) {
+  int hi = __double2hiint(x);
+  const int e = ((hi - 0x3fe6a09e) >> 20);
+  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
+  const double E = (double)e, p = a * E;
+  if (!(fabs(p) < 900.) || hi < 0x00100000 || hi >= 0x7ff00000) return pow(x, a);
+  const double n = rint(p);
+  const double r = fma((p - n) + fma(a, E, -p), 0.6931471805599453, a * log(m));
+  return ldexp(exp64<true>(r), (int)n);
+}
+
+// sqrt of v >= 0
+__device__ inline double sqrt_pos(double v) {
+  double ir;
+  return v > 1e-290 ? sqrt64(v, ir) : sqrt(v);
+}
+
 // TErnd_dft::spectrum (ternd_dft.cc:17-24)
 __device__ inline double spec_dft(double k, const hxg_ternd_dft_t &p) {
   if (k < p.k0) return 0.;
-  return p.rms * pow(k / p.k0, p.a0) / (4 * cgs::pi * k * k);
+  return p.rms * pow_k(k / p.k0, p.a0) / (4 * cgs::pi * k * k);
 }
 
 // Brnd_es::spectrum (brnd_es.cc:30-44)
@@ -94,35 +114,54 @@ __device__ inline double spec_es(double k, const hxg_brnd_es_t &p) {
   // evaluated
   double P = 0.;
   if (band1 != 0.)
-    P = band1 * pow(p.k0 / p.k1, p.a1) * pow(k / p.k1, 6.);
+    P = band1 * pow_k(p.k0 / p.k1, p.a1) * pow_k(k / p.k1, 6.);
   else if (band2 != 0.)
-    P = band2 / pow(k / p.k0, p.a1);
+    P = band2 / pow_k(k / p.k0, p.a1);
   else if (band3 != 0.)
-    P = band3 / pow(k / p.k0, p.a0);
+    P = band3 / pow_k(k / p.k0, p.a0);
   return P * p0 * unit;
 }
 
 // The square root of spatial_profile (ternd_dft.cc:26-33, brnd_es.cc:46-52),
 // exp(-r_cyl / r0) exp(-zz / z0), that both rescales take: one exponential
 // of half the summed exponent (equal to rounding).
+// ir0, iz0: 1/r0, 1/z0.
 __device__ inline double sqrt_profile(double x, double y, double z, const double obs[3],
-                                      double r0, double z0) {
-  const double r_cyl = sqrt(x * x + y * y) - fabs(obs[0]);
+                                      double ir0, double iz0) {
+  double ir;
+  const double r_cyl = sqrt64(fmax(x * x + y * y, 1e-280), ir) - fabs(obs[0]);
   const double zz = fabs(z) - fabs(obs[2]);
-  return exp(-0.5 * (r_cyl / r0 + zz / z0));
+  return exp64<true>(-0.5 * fma(r_cyl, ir0, zz * iz0));
 }
 
 struct RfgGrid {
   int nx, ny, nz;
   double lx, ly, lz, xmin, ymin, zmin;  // cm
   double dk3;                           // kpc^3 / (lx ly lz)
+  // k and vertex position of every index of the axes x, y, z, made once a call
+  // (rfg_axes_kernel): each costs one or two FP64 divisions
+  const double *kx, *ky, *kz, *vx, *vy, *vz;
 };
 
+__global__ void rfg_axes_kernel(RfgGrid G, double *out) {
+  const int n[3] = {G.nx, G.ny, G.nz}, all = G.nx + G.ny + G.nz;
+  const double len[3] = {G.lx, G.ly, G.lz}, lo[3] = {G.xmin, G.ymin, G.zmin};
+  int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= all) return;
+  const int at = i;
+  int a = 0;
+  while (i >= n[a]) i -= n[a++];
+  out[at] = kcomp(i, n[a], len[a]);
+  out[all + at] = i * len[a] / (n[a] - 1) + lo[a];
+}
+
+// Cell indices fit 32 bits (the host refuses larger grids): 64-bit divisions
+// would cost more than the rest of most of these kernels.
 __device__ inline void unflat(const RfgGrid &G, uint64_t idx, int &i, int &j, int &l) {
-  l = (int)(idx % G.nz);
-  const uint64_t t = idx / G.nz;
-  j = (int)(t % G.ny);
-  i = (int)(t / G.ny);
+  const unsigned n = (unsigned)idx, t = n / (unsigned)G.nz;
+  l = (int)(n - t * (unsigned)G.nz);
+  i = (int)(t / (unsigned)G.ny);
+  j = (int)(t - (unsigned)i * (unsigned)G.ny);
 }
 
 // ---- STEP I: Gaussian k-space fill ---------------------------------------
@@ -138,7 +177,8 @@ __global__ void rfg_fill_kernel(RfgGrid G, int kind, hxg_ternd_dft_t pt, hxg_brn
   }
   int i, j, l;
   unflat(G, idx, i, j, l);
-  const double kx = kcomp(i, G.nx, G.lx), ky = kcomp(j, G.ny, G.ly), kz = kcomp(l, G.nz, G.lz);
+  const double kx = __ldg(G.kx + i), ky = __ldg(G.ky + j), kz = __ldg(G.kz + l);
+  // correctly rounded: the spectra's bands begin at modes of the lattice
   const double ks = sqrt(kx * kx + ky * ky + kz * kz);
   double g[4];
   if (kind == 0)
@@ -146,37 +186,58 @@ __global__ void rfg_fill_kernel(RfgGrid G, int kind, hxg_ternd_dft_t pt, hxg_brn
   else
     gauss4<2>(seed, idx, g);
   if (kind == 0) {
-    const double sigma = sqrt(spec_dft(ks, pt) * G.dk3);
+    const double sigma = sqrt_pos(spec_dft(ks, pt) * G.dk3);
     c0[idx] = make_double2(sigma * g[0], sigma * g[1]);
   } else {
-    const double sigma = sqrt(0.333333333333333333 * spec_es(ks, pb) * G.dk3);
+    const double sigma = sqrt_pos(0.333333333333333333 * spec_es(ks, pb) * G.dk3);
     c0[idx] = make_double2(sigma * g[0], sigma * g[1]);
     c1[idx] = make_double2(sigma * g[2], sigma * g[3]);
   }
 }
 
 // ---- per-block partial sums of a double array (for mean and variance) ----
-__global__ void rfg_sum_kernel(const double *x, uint64_t n, double mean, int squared,
-                               double *partial) {
+constexpr int kParts = 1024;
+
+__device__ inline double block_sum(double acc) {
   __shared__ double sh[256];
-  double acc = 0.;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const double v = x[i] - mean;
-    acc += squared ? v * v : x[i];
-  }
   sh[threadIdx.x] = acc;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
+  return sh[0];
+}
+
+// sums of x, or with a mean of (x - mean)^2
+__global__ void rfg_sum_kernel(const double *x, uint64_t n, const double *mean,
+                               double *partial) {
+  const double m = mean ? *mean : 0.;
+  double acc = 0.;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const double v = x[i] - m;
+    acc += mean ? v * v : v;
+  }
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+}
+
+// out[0] = the kParts partial sums over n, out[1] = 1 / sqrt(scale out[0])
+__global__ void rfg_mean_kernel(const double *partial, uint64_t n, double scale, double *out) {
+  double acc = 0.;
+  for (int k = threadIdx.x; k < kParts; k += 256) acc += partial[k];
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) {
+    out[0] = acc / (double)n;
+    out[1] = 1. / sqrt(scale * out[0]);
+  }
 }
 
 // ---- STEP II (TErnd_dft): real part times the profile ratio ---------------
 __global__ void ternd_rescale_kernel(RfgGrid G, hxg_ternd_dft_t p, double obs0, double obs1,
-                                     double obs2, double var_invsq, const double2 *c,
+                                     double obs2, double ir0, double iz0, const double *isd,
+                                     const double2 *c,
                                      double *te) {
   const uint64_t n = (uint64_t)G.nx * G.ny * G.nz;
   const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -184,10 +245,10 @@ __global__ void ternd_rescale_kernel(RfgGrid G, hxg_ternd_dft_t p, double obs0, 
   int i, j, l;
   unflat(G, idx, i, j, l);
   const double obs[3] = {obs0, obs1, obs2};
-  const double x = i * G.lx / (G.nx - 1) + G.xmin;
-  const double y = j * G.ly / (G.ny - 1) + G.ymin;
-  const double z = l * G.lz / (G.nz - 1) + G.zmin;
-  const double ratio = sqrt_profile(x, y, z, obs, p.r0, p.z0) * p.rms * var_invsq;
+  const double x = __ldg(G.vx + i);
+  const double y = __ldg(G.vy + j);
+  const double z = __ldg(G.vz + l);
+  const double ratio = sqrt_profile(x, y, z, obs, ir0, iz0) * p.rms * __ldg(isd);
   te[idx] = c[idx].x * ratio;
 }
 
@@ -229,42 +290,80 @@ __device__ inline V3<double> breg_grid_at(const RfgBregGrid &g, double x, double
 // (brnd_es.cc:157-204).  A vertex where the regular field is zero (versor
 // length^2 below 1e-10) keeps the unscaled value of the first transform,
 // as in the reference.
+// Constants of the rescale: profile lengths, the factors of the components along
+// and across the regular field, and for the spiral sin and cos of its pitch with
+// the sign of its amplitude.
+struct AnisoConst {
+  double ir0, iz0, par, perp, sp_s, cp_s;
+  int spiral;
+};
+
+static AnisoConst aniso_const(const hxg_brnd_es_t &p, const DevModels &M, const hxg_grid_desc_t &g,
+                              bool gridded) {
+  AnisoConst A;
+  A.ir0 = 1. / p.r0;
+  A.iz0 = 1. / p.z0;
+  const double rho2 = p.rho * p.rho;
+  const double norm = 1. / sqrt(0.333333333333333333 * rho2 + 0.666666666666666667 / rho2);
+  A.par = p.rho * norm;
+  A.perp = norm / p.rho;
+  const double sgn = M.sp_b0 < 0. ? -1. : 1.;
+  A.sp_s = sgn * M.sp_sin;
+  A.cp_s = sgn * M.sp_cos;
+  // |exponent| below 250 in the whole box and a plain b0: the squared amplitude
+  // is neither 0 nor infinite
+  const auto far = [](double a, double b) { return fmax(fabs(a), fabs(b)); };
+  const double rm = far(g.x_min, g.x_max) + far(g.y_min, g.y_max) + M.sp_rsun;
+  const double zm = far(g.z_min, g.z_max);
+  A.spiral = !gridded && M.breg == kBregSpiral && rm < 250. * fabs(M.sp_rs) &&
+             zm < 50. * fabs(M.sp_hs) && fabs(M.sp_b0) > 1e-20 && fabs(M.sp_b0) < 1e20;
+  return A;
+}
+
 template <bool kExt>
 __global__ void brnd_rescale_kernel(RfgGrid G, hxg_brnd_es_t p, DevModels M,
-                                    const ExtModels *ext, RfgBregGrid bg, double var_invsq,
+                                    const ExtModels *ext, RfgBregGrid bg, AnisoConst A,
+                                    const double *isd,
                                     double2 *c0, double2 *c1) {
   const uint64_t n = (uint64_t)G.nx * G.ny * G.nz;
   const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   int i, j, l;
   unflat(G, idx, i, j, l);
-  const double x = i * G.lx / (G.nx - 1) + G.xmin;
-  const double y = j * G.ly / (G.ny - 1) + G.ymin;
-  const double z = l * G.lz / (G.nz - 1) + G.zmin;
-  const double ratio = sqrt_profile(x, y, z, M.obs, p.r0, p.z0) * p.rms * var_invsq;
+  const double x = __ldg(G.vx + i);
+  const double y = __ldg(G.vy + j);
+  const double z = __ldg(G.vz + l);
+  const double ratio = sqrt_profile(x, y, z, M.obs, A.ir0, A.iz0) * p.rms * __ldg(isd);
   const double2 a0 = c0[idx], a1 = c1[idx];
   const double b[3] = {a0.x * ratio, a0.y * ratio, a1.y * ratio};
   const double p3[3] = {x, y, z};
-  const V3<double> H = bg.bx ? breg_grid_at(bg, x, y, z) : breg_model_x<kExt>(M, ext, x, y, z, p3);
-  // Hamvec::versor (include/hamvec.h:176-186)
-  const double l2 = H.x * H.x + H.y * H.y + H.z * H.z;
   double h[3] = {0., 0., 0.};
-  if (l2 != 0.) {
-    const double inv = 1. / sqrt(l2);
-    h[0] = H.x * inv;
-    h[1] = H.y * inv;
-    h[2] = H.z * inv;
+  if (A.spiral) {
+    // the spiral's direction, without its amplitude (which does not vanish
+    // anywhere in the box: the host's condition for this branch)
+    double ir;
+    const double r = sqrt64(fmax(x * x + y * y, 1e-280), ir);
+    if (outside_annulus<double>(r, p3, M.kpc, 3., 20.)) return;
+    h[0] = ir * (A.sp_s * x - A.cp_s * y);
+    h[1] = ir * (A.sp_s * y + A.cp_s * x);
+  } else {
+    const V3<double> H =
+        bg.bx ? breg_grid_at(bg, x, y, z) : breg_model_x<kExt>(M, ext, x, y, z, p3);
+    // Hamvec::versor (include/hamvec.h:176-186)
+    const double l2 = H.x * H.x + H.y * H.y + H.z * H.z;
+    if (l2 != 0.) {
+      const double inv = l2 > 1e-290 ? rsqrt64(l2) : 1. / sqrt(l2);
+      h[0] = H.x * inv;
+      h[1] = H.y * inv;
+      h[2] = H.z * inv;
+    }
+    if (h[0] * h[0] + h[1] * h[1] + h[2] * h[2] < 1e-10) return;
   }
-  if (h[0] * h[0] + h[1] * h[1] + h[2] * h[2] < 1e-10) return;
-  const double rho = p.rho;
-  const double rho2 = rho * rho;
-  const double rhonorm = 1. / sqrt(0.333333333333333333 * rho2 + 0.666666666666666667 / rho2);
   const double hb = h[0] * b[0] + h[1] * b[1] + h[2] * b[2];
   double o[3];
   for (int a = 0; a < 3; ++a) {
     const double par = h[a] * hb;
-    const double perp = b[a] - par;
-    o[a] = (par * rho + perp / rho) * rhonorm;
+    o[a] = par * A.par + (b[a] - par) * A.perp;
   }
   c0[idx] = make_double2(o[0], o[1]);
   c1[idx] = make_double2(o[1], o[2]);
@@ -277,18 +376,13 @@ __device__ inline uint64_t sym_index(const RfgGrid &G, int i, int j, int l) {
 }
 
 // ---- Brnd_es STEP III: Hermitian part and divergence-free projection ------
-// (brnd_es.cc:196-245): gramschmidt() with the sqrt(3) factor, times sqrt(2)
-__global__ void brnd_project_kernel(RfgGrid G, const double2 *c0, const double2 *c1,
-                                    double *bx, double *by, double *bz) {
-  const uint64_t n = (uint64_t)G.nx * G.ny * G.nz;
-  const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n) return;
-  int i, j, l;
-  unflat(G, idx, i, j, l);
-  const uint64_t s = sym_index(G, i, j, l);
-  const double k[3] = {kcomp(i, G.nx, G.lx), kcomp(j, G.ny, G.ly), kcomp(l, G.nz, G.lz)};
-  const double b[3] = {0.5 * (c0[idx].x + c0[s].x), 0.5 * (c1[idx].x + c1[s].x),
-                       0.5 * (c1[idx].y + c1[s].y)};
+// (brnd_es.cc:196-256): gramschmidt() with the sqrt(3) factor, times sqrt(2),
+// packed for the backward transform as c0 = (bx, by), c1 = (by, bz).  A cell and
+// its mirror -k have the same Hermitian part; one thread takes both, so that
+// the arrays are read and written once, in place.
+__device__ inline void project_cell(const RfgGrid &G, int i, int j, int l, const double b[3],
+                                    double2 &c0, double2 &c1) {
+  const double k[3] = {__ldg(G.kx + i), __ldg(G.ky + j), __ldg(G.kz + l)};
   const double kk = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
   const double bb = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
   double f[3] = {b[0], b[1], b[2]};
@@ -297,18 +391,30 @@ __global__ void brnd_project_kernel(RfgGrid G, const double2 *c0, const double2 
     const double kb = k[0] * b[0] + k[1] * b[1] + k[2] * b[2];
     for (int a = 0; a < 3; ++a) f[a] = 1.7320508075688772935 * (b[a] - k[a] * kb * inv_k_mod);
   }
-  bx[idx] = 1.4142135623730950488 * f[0];
-  by[idx] = 1.4142135623730950488 * f[1];
-  bz[idx] = 1.4142135623730950488 * f[2];
+  const double r2 = 1.4142135623730950488;
+  c0 = make_double2(r2 * f[0], r2 * f[1]);
+  c1 = make_double2(r2 * f[1], r2 * f[2]);
 }
 
-// c0 = (bx, by), c1 = (by, bz)  (brnd_es.cc:247-256)
-__global__ void brnd_repack_kernel(uint64_t n, const double *bx, const double *by,
-                                   const double *bz, double2 *c0, double2 *c1) {
+__global__ void brnd_project_kernel(RfgGrid G, double2 *c0, double2 *c1) {
+  const uint64_t n = (uint64_t)G.nx * G.ny * G.nz;
   const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
-  c0[idx] = make_double2(bx[idx], by[idx]);
-  c1[idx] = make_double2(by[idx], bz[idx]);
+  int i, j, l;
+  unflat(G, idx, i, j, l);
+  const uint64_t s = sym_index(G, i, j, l);
+  if (s < idx) return;
+  const double2 a0 = c0[idx], a1 = c1[idx], s0 = c0[s], s1 = c1[s];
+  const double b[3] = {0.5 * (a0.x + s0.x), 0.5 * (a1.x + s1.x), 0.5 * (a1.y + s1.y)};
+  double2 o0, o1;
+  project_cell(G, i, j, l, b, o0, o1);
+  c0[idx] = o0;
+  c1[idx] = o1;
+  if (s == idx) return;
+  // the mirror's own k: an index n/2 of an even axis is its own mirror
+  project_cell(G, i ? G.nx - i : 0, j ? G.ny - j : 0, l ? G.nz - l : 0, b, o0, o1);
+  c0[s] = o0;
+  c1[s] = o1;
 }
 
 // final Hermitian part over N (brnd_es.cc:259-300)
@@ -320,10 +426,18 @@ __global__ void brnd_final_kernel(RfgGrid G, const double2 *c0, const double2 *c
   int i, j, l;
   unflat(G, idx, i, j, l);
   const uint64_t s = sym_index(G, i, j, l);
+  if (s < idx) return;
   const double inv = 1. / (double)n;
-  bx[idx] = 0.5 * (c0[idx].x + c0[s].x) * inv;
-  by[idx] = 0.5 * (c1[idx].x + c1[s].x) * inv;
-  bz[idx] = 0.5 * (c1[idx].y + c1[s].y) * inv;
+  const double2 a1 = c1[idx], s1 = c1[s];
+  const double x = 0.5 * (c0[idx].x + c0[s].x) * inv;
+  const double y = 0.5 * (a1.x + s1.x) * inv, z = 0.5 * (a1.y + s1.y) * inv;
+  bx[idx] = x;
+  by[idx] = y;
+  bz[idx] = z;
+  if (s == idx) return;
+  bx[s] = x;
+  by[s] = y;
+  bz[s] = z;
 }
 
 // ---- host side ---------------------------------------------------------
@@ -331,27 +445,19 @@ __global__ void brnd_final_kernel(RfgGrid G, const double2 *c0, const double2 *c
 static unsigned nblk(uint64_t n) { return (unsigned)((n + 255) / 256); }
 
 // variance of the first n doubles of x (toolkit::variance, include/toolkit.h:70-78)
+// into stat[2] and 1 / sqrt(scale variance) into stat[3] (the mean into stat[0]),
+// without a host round trip between its two sums
 static cudaError_t variance(cudaStream_t s, const double *x, uint64_t n, double *part,
-                            int nparts, double *out) {
-  double h[1024];
-  double sum = 0.;
-  rfg_sum_kernel<<<nparts, 256, 0, s>>>(x, n, 0., 0, part);
-  cudaError_t e = cudaMemcpyAsync(h, part, nparts * sizeof(double), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return e;
-  for (int k = 0; k < nparts; ++k) sum += h[k];
-  const double mean = sum / (double)n;
-  rfg_sum_kernel<<<nparts, 256, 0, s>>>(x, n, mean, 1, part);
-  e = cudaMemcpyAsync(h, part, nparts * sizeof(double), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return e;
-  double var = 0.;
-  for (int k = 0; k < nparts; ++k) var += h[k];
-  *out = var / (double)n;
-  return cudaSuccess;
+                            double scale, double *stat) {
+  rfg_sum_kernel<<<kParts, 256, 0, s>>>(x, n, nullptr, part);
+  rfg_mean_kernel<<<1, 256, 0, s>>>(part, n, 1., stat);
+  rfg_sum_kernel<<<kParts, 256, 0, s>>>(x, n, stat, part);
+  rfg_mean_kernel<<<1, 256, 0, s>>>(part, n, scale, stat + 2);
+  return cudaGetLastError();
 }
 
-static RfgGrid rfg_grid(const hxg_grid_desc_t &g) {
+// The grid's constants, its axis tables queued on s.
+static RfgGrid rfg_grid(cudaStream_t s, const hxg_grid_desc_t &g, double *axes) {
   RfgGrid G;
   G.nx = (int)g.nx;
   G.ny = (int)g.ny;
@@ -363,6 +469,14 @@ static RfgGrid rfg_grid(const hxg_grid_desc_t &g) {
   G.ymin = g.y_min;
   G.zmin = g.z_min;
   G.dk3 = cgs::kpc * cgs::kpc * cgs::kpc / (G.lx * G.ly * G.lz);
+  const int all = G.nx + G.ny + G.nz;
+  G.kx = axes;
+  G.ky = G.kx + G.nx;
+  G.kz = G.ky + G.ny;
+  G.vx = axes + all;
+  G.vy = G.vx + G.nx;
+  G.vz = G.vy + G.ny;
+  rfg_axes_kernel<<<(all + 255) / 256, 256, 0, s>>>(G, axes);
   return G;
 }
 
@@ -371,7 +485,7 @@ static RfgGrid rfg_grid(const hxg_grid_desc_t &g) {
 struct RfgWork {
   uint32_t nx = 0, ny = 0, nz = 0;
   double2 *c0 = nullptr, *c1 = nullptr;
-  double *part = nullptr;
+  double *part = nullptr, *axes = nullptr;
   cufftHandle plan = 0;
   bool have_plan = false;
   void release() {
@@ -379,6 +493,7 @@ struct RfgWork {
     if (c0) cudaFree(c0);
     if (c1) cudaFree(c1);
     if (part) cudaFree(part);
+    if (axes) cudaFree(axes);
     *this = RfgWork{};
   }
 };
@@ -419,7 +534,8 @@ static int rfg_setup(cudaStream_t s, const hxg_grid_desc_t &g, bool two, RfgWork
   if (W.nx != g.nx || W.ny != g.ny || W.nz != g.nz) {
     W.release();
     RFG_CK(cudaMalloc(&W.c0, n * sizeof(double2)));
-    RFG_CK(cudaMalloc(&W.part, 1024 * sizeof(double)));
+    RFG_CK(cudaMalloc(&W.part, (kParts + 4) * sizeof(double)));
+    RFG_CK(cudaMalloc(&W.axes, 2 * ((size_t)g.nx + g.ny + g.nz) * sizeof(double)));
     RFG_FFT(cufftPlan3d(&W.plan, (int)g.nx, (int)g.ny, (int)g.nz, CUFFT_Z2Z));
     W.have_plan = true;
     W.nx = g.nx;
@@ -431,13 +547,21 @@ static int rfg_setup(cudaStream_t s, const hxg_grid_desc_t &g, bool two, RfgWork
   return HXG_OK;
 }
 
+// Waits for the field and refuses one whose variance is zero or not finite.
+static int finish(cudaStream_t s, const double *d_var) {
+  double var = 0.;
+  RFG_CK(cudaMemcpyAsync(&var, d_var, sizeof(var), cudaMemcpyDeviceToHost, s));
+  RFG_CK(cudaStreamSynchronize(s));
+  return var > 0. && std::isfinite(var) ? HXG_OK : HXG_ERR_INVALID;
+}
+
 int generate_ternd_dft(cudaStream_t s, RfgWork *&work, const hxg_grid_desc_t &g,
                        const hxg_ternd_dft_t &p, const double obs[3], uint64_t seed,
                        double *te) {
   int st = rfg_setup(s, g, false, work);
   if (st != HXG_OK) return st;
   RfgWork &W = *work;
-  const RfgGrid G = rfg_grid(g);
+  const RfgGrid G = rfg_grid(s, g, W.axes);
   const uint64_t n = (uint64_t)g.nx * g.ny * g.nz;
   const hxg_brnd_es_t none{};
   rfg_fill_kernel<<<nblk(n), 256, 0, s>>>(G, 0, p, none, seed, W.c0, nullptr);
@@ -445,14 +569,12 @@ int generate_ternd_dft(cudaStream_t s, RfgWork *&work, const hxg_grid_desc_t &g,
   RFG_FFT(cufftExecZ2Z(W.plan, W.c0, W.c0, CUFFT_INVERSE));
   // the reference's variance runs over the first n doubles of the complex
   // array, i.e. the interleaved (Re, Im) of its first n/2 cells
-  double var = 0.;
-  RFG_CK(variance(s, reinterpret_cast<const double *>(W.c0), n, W.part, 1024, &var));
-  if (!(var > 0.) || !std::isfinite(var)) return HXG_ERR_INVALID;
-  const double var_invsq = 1. / sqrt(var);
-  ternd_rescale_kernel<<<nblk(n), 256, 0, s>>>(G, p, obs[0], obs[1], obs[2], var_invsq, W.c0, te);
+  double *const stat = W.part + kParts;
+  RFG_CK(variance(s, reinterpret_cast<const double *>(W.c0), n, W.part, 1., stat));
+  ternd_rescale_kernel<<<nblk(n), 256, 0, s>>>(G, p, obs[0], obs[1], obs[2], 1. / p.r0,
+                                               1. / p.z0, stat + 3, W.c0, te);
   RFG_CK(cudaGetLastError());
-  RFG_CK(cudaStreamSynchronize(s));
-  return HXG_OK;
+  return finish(s, stat + 2);
 }
 
 int generate_brnd_es(cudaStream_t s, RfgWork *&work, const hxg_grid_desc_t &g,
@@ -462,35 +584,32 @@ int generate_brnd_es(cudaStream_t s, RfgWork *&work, const hxg_grid_desc_t &g,
   int st = rfg_setup(s, g, true, work);
   if (st != HXG_OK) return st;
   RfgWork &W = *work;
-  const RfgGrid G = rfg_grid(g);
+  const RfgGrid G = rfg_grid(s, g, W.axes);
   const uint64_t n = (uint64_t)g.nx * g.ny * g.nz;
   const hxg_ternd_dft_t none{};
   rfg_fill_kernel<<<nblk(n), 256, 0, s>>>(G, 1, none, p, seed, W.c0, W.c1);
   RFG_CK(cudaGetLastError());
   RFG_FFT(cufftExecZ2Z(W.plan, W.c0, W.c0, CUFFT_INVERSE));
   RFG_FFT(cufftExecZ2Z(W.plan, W.c1, W.c1, CUFFT_INVERSE));
-  double var = 0.;
-  RFG_CK(variance(s, reinterpret_cast<const double *>(W.c0), n, W.part, 1024, &var));
-  if (!(var > 0.) || !std::isfinite(var)) return HXG_ERR_INVALID;
-  const double var_invsq = 1. / sqrt(3. * var);
+  double *const stat = W.part + kParts;
+  RFG_CK(variance(s, reinterpret_cast<const double *>(W.c0), n, W.part, 3., stat));
+  const AnisoConst A = aniso_const(p, M, g, breg.bx != nullptr);
   if (ext)
-    brnd_rescale_kernel<true><<<nblk(n), 256, 0, s>>>(G, p, M, ext, breg, var_invsq, W.c0, W.c1);
+    brnd_rescale_kernel<true><<<nblk(n), 256, 0, s>>>(G, p, M, ext, breg, A, stat + 3, W.c0,
+                                                      W.c1);
   else
-    brnd_rescale_kernel<false><<<nblk(n), 256, 0, s>>>(G, p, M, ext, breg, var_invsq, W.c0,
-                                                       W.c1);
+    brnd_rescale_kernel<false><<<nblk(n), 256, 0, s>>>(G, p, M, ext, breg, A, stat + 3, W.c0,
+                                                      W.c1);
   RFG_CK(cudaGetLastError());
   RFG_FFT(cufftExecZ2Z(W.plan, W.c0, W.c0, CUFFT_FORWARD));
   RFG_FFT(cufftExecZ2Z(W.plan, W.c1, W.c1, CUFFT_FORWARD));
-  brnd_project_kernel<<<nblk(n), 256, 0, s>>>(G, W.c0, W.c1, bx, by, bz);
-  RFG_CK(cudaGetLastError());
-  brnd_repack_kernel<<<nblk(n), 256, 0, s>>>(n, bx, by, bz, W.c0, W.c1);
+  brnd_project_kernel<<<nblk(n), 256, 0, s>>>(G, W.c0, W.c1);
   RFG_CK(cudaGetLastError());
   RFG_FFT(cufftExecZ2Z(W.plan, W.c0, W.c0, CUFFT_INVERSE));
   RFG_FFT(cufftExecZ2Z(W.plan, W.c1, W.c1, CUFFT_INVERSE));
   brnd_final_kernel<<<nblk(n), 256, 0, s>>>(G, W.c0, W.c1, bx, by, bz);
   RFG_CK(cudaGetLastError());
-  RFG_CK(cudaStreamSynchronize(s));
-  return HXG_OK;
+  return finish(s, stat + 2);
 }
 
 }  // namespace hxg
