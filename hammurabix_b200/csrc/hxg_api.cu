@@ -88,6 +88,7 @@ struct hxg_handle {
   std::map<uint64_t, DevBuf> interp;
   size_t interp_bytes = 0;
   size_t interp_limit = 8ull << 30;
+  DevBuf part;  // per-lane sums of FP32C launches (part_sums)
   DevBuf out;  // device maps of the host-buffer calls
   // pinned landing zone of small host-buffer calls (kLanding bytes, on first use)
   char *landing = nullptr;
@@ -1033,6 +1034,7 @@ int hxg_destroy(hxg_handle *h) {
   if (h->shell_all.p) cudaFree(h->shell_all.p);
   for (auto &kv : h->interp) cudaFree(kv.second.p);
   if (h->out.p) cudaFree(h->out.p);
+  if (h->part.p) cudaFree(h->part.p);
   if (h->landing) cudaFreeHost(h->landing);
   for (auto &b : h->ck)
     if (b.p) cudaFree(b.p);
@@ -1460,6 +1462,32 @@ unsigned shard_block_log2(uint64_t npix, uint32_t nshards) {
   return L;
 }
 
+// Whether rays of a launch can leave the cuts within their first 0.4.  A lone
+// FP32C adjoint shell to 30 kpc, cut from 0.33 on, takes 13.9 ms with a chunk per
+// block against 16.7; one to 20 kpc, cut from 0.5 on, 4.05 against 3.8 ms, so
+// it keeps a pixel's chunks in one warp.
+bool cut_early(const ShellLaunch &F) {
+  double r2 = 0.;
+  for (int k = 0; k < 3; ++k) r2 += F.obs[k] * F.obs[k];
+  const double reach = std::min(F.gc_r_max - std::sqrt(r2),
+                                std::min(F.gc_z_max - F.obs[2], F.obs[2] - F.gc_z_min));
+  return reach < F.d_start + 0.4 * F.delta * (double)F.step;
+}
+
+// Lets an FP32C launch of `lanes` lanes and nf passes take one chunk per block
+// (P.part) where half of a warp's chunks would idle past the cuts: shells cut
+// early, with more lanes than the device holds at a time.  The sums are the same
+// bits.  Off when the device has no room for them.
+void part_sums(hxg_handle *h, ShellLaunch &P, uint64_t lanes, int nf) {
+  if (P.chunks == 1 || lanes < 896ull * h->sm_count || !cut_early(P)) return;
+  if (ensure(h, h->part, lanes * (2 + 3 * nf) * sizeof(double)) != HXG_OK) {
+    (void)cudaGetLastError();
+    return;
+  }
+  P.part = static_cast<double *>(h->part.p);
+  P.part_n = lanes;
+}
+
 // Shell s of pass o over the pixels of shard `shard` of `nshards` (the
 // 32-pixel NESTED blocks b with b % nshards == shard) into the shell maps tmp (radial_integration for every pixel of the shell,
 // integrator.cc:60-100); fdmap = the accumulated FD output of the inner
@@ -1513,6 +1541,7 @@ int run_shell(hxg_handle *h, const hxg_obs_t &o, uint32_t s, const ExtModels *ex
   const uint64_t warps = (local + (32 / C) - 1) / (32 / C);
   const unsigned threads = fp32 ? HXG_FP32C_THREADS : HXG_FP64_THREADS;
   const unsigned blocks = (unsigned)((warps * 32 + threads - 1) / threads);
+  if (fp32) part_sums(h, P, local * C, 1);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->timing) {
     HXG_CK(cudaEventCreate(&e0));
@@ -1520,7 +1549,7 @@ int run_shell(hxg_handle *h, const hxg_obs_t &o, uint32_t s, const ExtModels *ex
     HXG_CK(cudaEventRecord(e0, h->stream));
   }
   HXG_CK(launch_shell(h->stream, fp32, P, blocks, threads));
-  ++h->launch_count;
+  h->launch_count += P.part ? 2 : 1;
   if (h->timing) {
     HXG_CK(cudaEventRecord(e1, h->stream));
     h->events.emplace_back(e0, e1);
@@ -1815,6 +1844,7 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
   const bool fp32 = h->precision == HXG_FP32C;
   const unsigned threads = fp32 ? HXG_FP32C_MULTI_THREADS : HXG_FP64_THREADS;
   const unsigned blocks = (unsigned)((warps * 32 + threads - 1) / threads);
+  if (fp32) part_sums(h, P, local * C, NF);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->timing) {
     HXG_CK(cudaEventCreate(&e0));
@@ -1822,7 +1852,7 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
     HXG_CK(cudaEventRecord(e0, h->stream));
   }
   HXG_CK(launch_shell_multi(h->stream, fp32, P, NF, &Fq, blocks, threads));
-  ++h->launch_count;
+  h->launch_count += P.part ? 2 : 1;
   if (h->timing) {
     HXG_CK(cudaEventRecord(e1, h->stream));
     h->events.emplace_back(e0, e1);
@@ -2169,17 +2199,9 @@ int adjoint_shell(hxg_handle *h, const hxg_obs_t &o, uint32_t s, uint32_t shard,
   if (local == 0) return HXG_OK;
   const uint64_t warps = (local + (32 / C) - 1) / (32 / C);
   const unsigned threads = fp32 ? HXG_ADJ32_THREADS : HXG_ADJ_THREADS;
-  // FP32C: whole blocks of pixels for each chunk in shells whose rays can
-  // leave the cuts in their first 0.4 (hxg_adjoint32.cuh): a lone shell to 30
-  // kpc, cut from 0.33 on, 13.9 against 16.7 ms; one to 20 kpc, cut from 0.5 on,
-  // 4.05 against 3.8 ms, so it keeps the mapping of the forward
-  if (fp32 && C > 1) {
-    double mid = F.d_start + 0.4 * F.delta * (double)F.step, r2 = 0.;
-    for (int k = 0; k < 3; ++k) r2 += F.obs[k] * F.obs[k];
-    const double reach = std::min(F.gc_r_max - std::sqrt(r2),
-                                  std::min(F.gc_z_max - F.obs[2], F.obs[2] - F.gc_z_min));
-    A.by_chunk = reach < mid;
-  }
+  // FP32C: whole blocks of pixels for each chunk in shells whose rays can be cut
+  // early (hxg_adjoint32.cuh)
+  A.by_chunk = fp32 && C > 1 && cut_early(F);
   const unsigned blocks = A.by_chunk ? (unsigned)((local + threads - 1) / threads * C)
                                      : (unsigned)((warps * 32 + threads - 1) / threads);
   HXG_CK(fp32 ? launch_adjoint32(h->stream, A, blocks, threads)

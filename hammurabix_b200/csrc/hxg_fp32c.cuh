@@ -219,6 +219,35 @@ __device__ __forceinline__ float cre_ana_prof32(const FastModels &F, float rf, f
   return __fdividef(ex2_approx(fmaf(-rf, F.cre_ir0_l2, F.cre_R0_l2)) * t, den * den);
 }
 
+// The end of a pixel, by its C lanes: checkpoint, chunk combination, shell maps.
+template <int NF>
+__device__ __forceinline__ void finish_pixel(const ShellLaunch &P, const FreqSet<NF> &Fq,
+                                             bool valid, bool live, unsigned long long nest,
+                                             uint64_t ring, int c, double dm, double fd,
+                                             double si[NF], double sq[NF], double su[NF]) {
+  if (NF == 1 && P.ck != nullptr) store_checkpoint(P, live, nest, c, 1, fd, sq[0], su[0]);
+  combine_chunks_nf<NF>(P, Fq, c, dm, fd, si, sq, su);
+  if (live && c == 0) {
+    if (P.do_dm) P.out[0][ring] = dm;
+    if (P.do_fd || P.do_sync) P.out[1][ring] = fd;
+    if (P.do_sync) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        Fq.out[f][0][ring] = si[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+        Fq.out[f][1][ring] = sq[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+        Fq.out[f][2][ring] = su[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
+      }
+    }
+  } else if (valid && !live && c == 0) {
+    if (P.do_dm) P.out[0][ring] = 0.;
+    if (P.do_fd || P.do_sync) P.out[1][ring] = 0.;
+    if (P.do_sync) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) Fq.out[f][0][ring] = Fq.out[f][1][ring] = Fq.out[f][2][ring] = 0.;
+    }
+  }
+}
+
 // Warp gw of shell launch P (32/C pixels, C lanes each) for the NF
 // frequency passes of Fq.  All 32 lanes of the warp call it with the same gw.
 // kFast: the launch's models are among B none/grid/spiral, n_e
@@ -228,12 +257,20 @@ __device__ __forceinline__ float cre_ana_prof32(const FastModels &F, float rf, f
 template <int NG, bool kExt, int NF, bool kFast = false>
 __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<NF> &Fq,
                                            long long gw, int lane) {
-  const int C = P.chunks;
-  const int seg = lane >> P.log2_chunks;
-  const int c = lane & (C - 1);
+  // 32/C pixels side by side with their C chunks each, or (part) 32 pixels of
+  // one chunk: warps of chunk 0 of every pixel, then of chunk 1, ...
   const Hpx h = hpx_make((uint64_t)P.nside);
-  const unsigned long long nest =
-      shard_nest(P, (unsigned long long)gw * (32 >> P.log2_chunks) + seg);
+  unsigned long long local = (unsigned long long)gw * 32 + lane;
+  int c = (int)(local & (unsigned)(P.chunks - 1));
+  if (P.part != nullptr) {
+    const unsigned long long per = P.part_n >> P.log2_chunks;
+    c = (int)(local / per);
+    if (c >= P.chunks) return;
+    local -= (unsigned long long)c * per;
+  } else {
+    local >>= P.log2_chunks;
+  }
+  const unsigned long long nest = shard_nest(P, local);
   const bool valid = nest < h.npix;
   uint64_t ring = 0;
   bool live = false;
@@ -555,27 +592,19 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
       su[f] = ku[f].value() * Fq.k_p[f];
     }
   }
-  if (NF == 1 && P.ck != nullptr) store_checkpoint(P, live, nest, c, 1, fd, sq[0], su[0]);
-  combine_chunks_nf<NF>(P, Fq, c, dm, fd, si, sq, su);
-  if (live && c == 0) {
-    if (P.do_dm) P.out[0][ring] = dm;
-    if (P.do_fd || P.do_sync) P.out[1][ring] = fd;
-    if (P.do_sync) {
+  if (P.part != nullptr) {
+    double *const p = P.part + (local << P.log2_chunks) + c;
+    p[0] = dm;
+    p[P.part_n] = fd;
 #pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        Fq.out[f][0][ring] = si[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
-        Fq.out[f][1][ring] = sq[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
-        Fq.out[f][2][ring] = su[f] * Fq.tc_a[f] * Fq.tc_a[f] / Fq.tc_b[f];
-      }
+    for (int f = 0; f < NF; ++f) {
+      p[(2 + 3 * f) * P.part_n] = si[f];
+      p[(3 + 3 * f) * P.part_n] = sq[f];
+      p[(4 + 3 * f) * P.part_n] = su[f];
     }
-  } else if (valid && !live && c == 0) {
-    if (P.do_dm) P.out[0][ring] = 0.;
-    if (P.do_fd || P.do_sync) P.out[1][ring] = 0.;
-    if (P.do_sync) {
-#pragma unroll
-      for (int f = 0; f < NF; ++f) Fq.out[f][0][ring] = Fq.out[f][1][ring] = Fq.out[f][2][ring] = 0.;
-    }
+    return;
   }
+  finish_pixel<NF>(P, Fq, valid, live, nest, ring, c, dm, fd, si, sq, su);
 }
 
 // One frequency pass: the pass's constants from its launch block.
@@ -603,6 +632,38 @@ __global__ void __launch_bounds__(HXG_FP32C_MULTI_THREADS,
 shell_fp32c_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
   fp32c_tile<NG, kExt, NF, kFast>(P, Fq, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                            threadIdx.x & 31);
+}
+
+// The second half of a launch whose lanes left their sums in P.part: the
+// chunk combination in the mapping, and so with the sums, of a launch that
+// keeps a pixel's chunks in one warp.
+template <int NF>
+__global__ void __launch_bounds__(256) shell_combine_kernel(const ShellLaunch P,
+                                                            const FreqSet<NF> Fq) {
+  const unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = (int)(t & (unsigned)(P.chunks - 1));
+  const Hpx h = hpx_make((uint64_t)P.nside);
+  const unsigned long long nest = shard_nest(P, t >> P.log2_chunks);
+  const bool valid = t < P.part_n && nest < h.npix;
+  uint64_t ring = 0;
+  bool live = false;
+  double dm = 0., fd = 0., si[NF], sq[NF], su[NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) si[f] = sq[f] = su[f] = 0.;
+  if (valid) {
+    ring = hpx_nest2ring(h, nest);
+    live = (P.mask == nullptr) || (P.mask[ring] != 0);
+    const double *const p = P.part + t;
+    dm = p[0];
+    fd = p[P.part_n];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      si[f] = p[(2 + 3 * f) * P.part_n];
+      sq[f] = p[(3 + 3 * f) * P.part_n];
+      su[f] = p[(4 + 3 * f) * P.part_n];
+    }
+  }
+  finish_pixel<NF>(P, Fq, valid, live, nest, ring, c, dm, fd, si, sq, su);
 }
 
 }  // namespace hxg

@@ -93,6 +93,10 @@ struct ShellLaunch {
   double *ck;
   double *ck_inner;
   FastModels fast;
+  // FP32C: per-lane sums instead of maps (shell_combine_kernel finishes them),
+  // a block of the launch taking one chunk of its neighbouring pixels; null = off
+  double *part;
+  unsigned long long part_n;  // lanes of the launch (the sums' stride)
   // FP64 form: every exponent of the FastModels is below 680 in size; FP32C:
   // its constants are finite (the kFast instantiations need it)
   int fast_ok;
@@ -153,7 +157,7 @@ struct FreqSet {
 };
 
 // One pass's constants from its launch block.
-__device__ __forceinline__ void freq_of_launch(const ShellLaunch &P, FreqSet<1> &Fq) {
+__host__ __device__ __forceinline__ void freq_of_launch(const ShellLaunch &P, FreqSet<1> &Fq) {
   Fq.lambda2[0] = P.lambda2;
   Fq.phase_k[0] = P.phase_k;
   Fq.quarter_k[0] = P.quarter_k;

@@ -495,6 +495,11 @@ cudaError_t launch_shell(cudaStream_t s, bool fp32, const ShellLaunch &P,
       shell_fp32c_kernel<NG, false, true><<<blocks, threads, 0, s>>>(P);
     else
       shell_fp32c_kernel<NG, E, false><<<blocks, threads, 0, s>>>(P);
+    if (P.part) {
+      FreqSet<1> Fq;
+      freq_of_launch(P, Fq);
+      shell_combine_kernel<1><<<blocks_for(P.part_n, 256), 256, 0, s>>>(P, Fq);
+    }
   });
 }
 
@@ -515,6 +520,10 @@ cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, 
       shell_fp32c_multi_kernel<NG, E, 2, false><<<blocks, threads, 0, s>>>(P, F2);
     else
       shell_fp32c_multi_kernel<NG, E, 3, false><<<blocks, threads, 0, s>>>(P, F3);
+    if (P.part && nf == 2)
+      shell_combine_kernel<2><<<blocks_for(P.part_n, 256), 256, 0, s>>>(P, F2);
+    else if (P.part)
+      shell_combine_kernel<3><<<blocks_for(P.part_n, 256), 256, 0, s>>>(P, F3);
   });
 }
 
