@@ -181,6 +181,14 @@ def sub_workload_text(wl):
             f"Integrator::write_grid only")
 
 
+def reference_missing():
+    """Why the reference integrator cannot run here, or None."""
+    so = os.path.join(ROOT, "oracle", "_ref", "libhxref.so")
+    return None if os.path.exists(so) else (
+        "oracle/_ref/libhxref.so is not built (oracle/Makefile compiles it from the hammurabiX "
+        "sources, which are not on this host)")
+
+
 def cpu_baseline(wl, host_fields, steps=1):
     """The reference's FP64 OpenMP integrator (oracle/_ref, compiled from the
     reference sources) on the bounded sample (sub_workload), all host cores:
@@ -227,6 +235,9 @@ def run_reference_arm(args, wl):
     from hammurabix_b200 import workloads as W
     ws, rank, _ = replicas.env()
     if rank != 0:
+        return
+    if reference_missing():
+        print(json.dumps({"impl": "reference", "unavailable": reference_missing()}), flush=True)
         return
     b = W.random_grids_torch(wl["grid_n"], *wl["seeds"], device="cpu")
     host = [t.double().numpy().reshape(-1) for t in b]
@@ -515,7 +526,7 @@ def main():
 
     def step(ig, outs):
         """One config-3 step: the frequency passes in the Pipeline's order,
-        fused into one traversal per shell where the form allows (FP32C)."""
+        fused into one traversal per shell (shards: in the FP32C form)."""
         if shard:
             sharded.write_passes_sharded(ig, passes, [dict(zip(sharded.MAPS, m)) for m in outs],
                                          shell_tmp, rank, ws, reduce_sum, reduce_root)
@@ -587,9 +598,15 @@ def main():
         k64ms, _, k64s = ig64.get_timing()
         ig64.set_timing(False)
         ms64 = t64 / args.fp64_steps * 1e3
+        ms64_1 = None
+        if not shard:
+            step_one_by_one(ig64, out64)
+            ms64_1 = max_over_ranks(timed(ig64, out64, args.fp64_steps,
+                                          step_one_by_one)) / args.fp64_steps * 1e3
         fp64 = {"ms_per_step": ms64, "ms_per_map": ms64 / len(passes),
                 "samples_per_s": (1 if shard else ws) * samples_step / (ms64 / 1e3),
-                "kernel_samples_per_s": k64s / (k64ms / 1e3) if k64ms > 0 else None}
+                "kernel_samples_per_s": k64s / (k64ms / 1e3) if k64ms > 0 else None,
+                "passes_one_by_one_ms": ms64_1}
         # errors of the last pass (0.408 GHz, sync only) and of the first
         # pass's DM/FD: rerun pass 0 and the last pass in both forms
         errs = {}
@@ -831,7 +848,9 @@ def main():
 
     cpu = None
     # the CPU reference is timed at N = 1 only (the other ranks would wait)
-    if rank == 0 and ws == 1 and not args.no_cpu_baseline:
+    if rank == 0 and ws == 1 and not args.no_cpu_baseline and reference_missing():
+        cpu = {"unavailable": reference_missing()}
+    elif rank == 0 and ws == 1 and not args.no_cpu_baseline:
         host = [t.cpu().numpy() for t in f64]
         cb = cpu_baseline(wl, host)
         v = cb["samples"] / cb["seconds"][0]
@@ -853,11 +872,10 @@ def main():
             "ms_per_map": ms_step / len(passes),
             "fp64": fp64,
             "fp32c_passes_one_by_one": one_by_one,
-            # the product step (passes fused into one traversal per shell)
-            # against the plain FP64 form, and the precision change alone
-            # (both forms pass by pass)
+            # the product step (passes fused into one traversal per shell) of
+            # the two forms, and the precision change alone (pass by pass)
             "fp32c_speedup_vs_fp64": (fp64["ms_per_step"] / ms_step) if fp64 else None,
-            "fp32c_precision_speedup_vs_fp64": (fp64["ms_per_step"] / one_by_one["ms_per_step"]
+            "fp32c_precision_speedup_vs_fp64": (fp64["passes_one_by_one_ms"] / one_by_one["ms_per_step"]
                                                 if fp64 and one_by_one else None),
             "fp32c_max_rel_err_vs_fp64": errs,
             "adjoint_fwd_ratio": adjoint["ratio"] if adjoint else None,
