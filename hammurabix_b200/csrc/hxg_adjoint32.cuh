@@ -152,8 +152,8 @@ shell_fp32c_adjoint_kernel(const AdjointLaunch A) {
       gvy = uy * G.scale[1];
       gvz = uz * G.scale[2];
     }
-    long long wlo, whi, slo_unused, shi_unused;
-    ray_window(P, ux, uy, uz, wlo, whi, slo_unused, shi_unused);
+    long long wlo, whi;
+    ray_window(P, ux, uy, uz, wlo, whi);
     exact_cut_window(P, uz, ou2, oo, wlo, whi);
     const int i0 = (int)max((P.step * c) >> P.log2_chunks, wlo);
     const int i1 = (int)min((P.step * (c + 1)) >> P.log2_chunks, whi);

@@ -99,7 +99,7 @@ struct hxg_handle {
   int64_t acc_launches = 0, acc_samples = 0;
   double waves = 4.0;
   int64_t launch_count = 0;
-  // adjoint checkpoint of the last forward pass (FP64 form)
+  // adjoint checkpoint of the last forward pass
   bool checkpoint = false;
   bool ck_valid = false;
   hxg_obs_t ck_obs{};
@@ -732,7 +732,6 @@ int build_launch(hxg_handle *h, const hxg_models_t &m, const hxg_obs_t &o,
       P.em_gp = std::tgamma(-0.25 * idx + 7. / 12.) * std::tgamma(-0.25 * idx - 1. / 12.);
       P.em_den_t = 4. * cgs::pi * mec2 * (1. - idx);
       const double e = 0.5 * (idx + 1);
-      P.em_pow_kind = (e == -1.) ? 1 : (e == 0. ? 2 : 0);
       P.em_pe = 1. - e;
       const double ae = std::pow(a_s, e);
       P.k_t = kbase / P.em_den_t * ae * P.em_gt * delta * P.i2bt;

@@ -348,8 +348,8 @@ __device__ __forceinline__ void fp32c_tile(const ShellLaunch &P, const FreqSet<N
     const double rc2_hi = F.rc2_hi, rc2_lo = F.rc2_lo;
     float last_index = __int_as_float(0x7fc00000), gt = float(P.em_gt),
           gp = float(P.em_gp), inv1mi = 1.f;
-    long long wlo, whi, slo_unused, shi_unused;
-    ray_window(P, ux, uy, uz, wlo, whi, slo_unused, shi_unused);
+    long long wlo, whi;
+    ray_window(P, ux, uy, uz, wlo, whi);
     // kFast: no inner radius, so the window is cut to the passing samples
     if (kFast) exact_cut_window(P, uz, ou2, oo, wlo, whi);
     // sample indices fit 32 bits (step < 2^31, checked on the host)

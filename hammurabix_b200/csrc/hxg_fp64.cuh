@@ -78,8 +78,8 @@ __device__ __forceinline__ void chunk_range64(const ShellLaunch &P, const double
     const double len = sqrt(px * px + py * py + pz * pz);
     return !(len > P.gc_r_max || pz < P.gc_z_min || pz > P.gc_z_max);
   };
-  long long lo, hi, slo_unused, shi_unused;
-  ray_window(P, u[0], u[1], u[2], lo, hi, slo_unused, shi_unused);
+  long long lo, hi;
+  ray_window(P, u[0], u[1], u[2], lo, hi);
   while (lo < hi && !pass(lo)) ++lo;
   while (hi > lo && !pass(hi - 1)) --hi;
   // sample indices fit 32 bits (checked on the host)

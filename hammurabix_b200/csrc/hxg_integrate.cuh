@@ -73,7 +73,6 @@ struct ShellLaunch {
   double tc_a, tc_b;         // temp_convert(t) = t*a*a/b (integrator.cc:275-279)
   // analytic synchrotron emissivity (integrator.cc:332-346, 401-415)
   int em_const;              // spectral index constant over space
-  int em_pow_kind;           // 0: pow(); 1: exponent == -1; 2: exponent == 0
   double em_index;           // constant index
   double em_n0u;             // j0 * gamma0^-index(observer) * unit
   double em_qe3, em_den_t, em_den_p, em_anum, em_3qe;
@@ -186,21 +185,16 @@ __device__ __forceinline__ unsigned long long shard_nest(const ShellLaunch &P,
 // spherical |pos| <= r_max and vertical z_min <= z <= z_max cuts
 // (integrator.cc:179-182), from the roots of |o + u d|^2 = r_max^2 and
 // o_z + u_z d = z_min / z_max, widened by two samples on each side.  Samples
-// outside the window fail the cuts; the samples of [slo, shi) lie two or
-// more steps inside it and pass them for certain, the others inside the
-// window are tested exactly, so the result is the per-sample test's.
+// outside the window fail the cuts; the callers test the others.
 __device__ __forceinline__ void ray_window(const ShellLaunch &P, double ux,
-                                           double uy, double uz,
-                                           long long &lo, long long &hi,
-                                           long long &slo, long long &shi) {
+                                           double uy, double uz, long long &lo,
+                                           long long &hi) {
   const double ox = P.obs[0], oy = P.obs[1], oz = P.obs[2];
   const double b = ox * ux + oy * uy + oz * uz;  // o.u
   const double c = (ox * ox + oy * oy + oz * oz) - P.gc_r_max * P.gc_r_max;
   const double disc = b * b - c;
   lo = 0;
   hi = 0;
-  slo = 0;
-  shi = 0;
   if (!(disc >= 0.)) return;  // the ray misses the r_max sphere
   const double sq = sqrt(disc);
   double da = -b - sq, db = -b + sq;
@@ -221,14 +215,6 @@ __device__ __forceinline__ void ray_window(const ShellLaunch &P, double ux,
   const double fb = fmin(fmax(ceil(xb) + 3., 0.), n);
   lo = (long long)fa;
   hi = (long long)fb;
-  // samples two or more steps inside both ends pass the cuts for certain
-  // (the rounding of da, db and of the sample positions is ~1e-12 of a
-  // step); with an inner radius the ray may cross the r_min ball, so every
-  // sample is tested
-  if (!(P.gc_r_min > 0.)) {
-    slo = (long long)fmin(fmax(ceil(xa) + 2., 0.), n);
-    shi = (long long)fmin(fmax(floor(xb) - 1., 0.), n);
-  }
 }
 
 // Sample range [ga, gb) of [i0, i1) in which the ray can be inside the grid
