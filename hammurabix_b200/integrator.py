@@ -202,8 +202,8 @@ class Integrator:
     def write_grid_multi_device(self, passes):
         """Several frequency passes at once (hxg_write_grid_multi): passes is
         a list of (obs, [dm, fd, is, qs, us]) with torch CUDA float64 tensors
-        (None where the pass writes no such map).  In the FP32C form up to
-        three passes with the same geometry share one traversal per shell."""
+        (None where the pass writes no such map).  Up to three passes
+        with the same geometry share one traversal per shell."""
         n = len(passes)
         obs = (abi.Obs * n)(*[o for o, _ in passes])
         ptrs = (C.c_void_p * (5 * n))()

@@ -71,8 +71,8 @@ class Pipeline:
             self.assemble_fields()
         self.maps = {}
         self.raw = []
-        # all passes in one call: the FP32C form runs passes of the same
-        # geometry in one traversal per shell (hxg_write_grid_multi)
+        # all passes in one call: passes of the same geometry share one
+        # traversal per shell (hxg_write_grid_multi)
         obs = [par.obs_pass(k) for k in range(par.num_passes())]
         outs = self.integ.write_grid_multi(obs)
         for k, (o, out) in enumerate(zip(obs, outs)):
