@@ -223,17 +223,20 @@ __device__ __forceinline__ void jf12_field(const Jf12Dev &J, double x, double y,
   const double rc_X = fma(az, J.cot_x, J.p.rpc_X);
   double rp_X, B_X, cX = J.cos_x, sX = J.sin_x;
   if (r < rc_X) {
-    const double q = J.p.rpc_X * rcp64(rc_X);
-    rp_X = r * q;
+    // a division as in the reference: rc_X is infinite for Xtheta = 0, and near
+    // the plane r - rp_X is all cancellation
+    rp_X = r * J.p.rpc_X / rc_X;
+    const double q = rp_X * ir;
     B_X = q * q;
-    // the angle's tangent is |z| / (r - rp_X); a right angle in the plane
+    // cos and sin of atan(|z| / (r - rp_X)), which is negative where rp_X is
+    // beyond r (rc_X below rpc_X); a right angle in the plane
     const double a = r - rp_X, h2 = fma(a, a, az * az);
     cX = 0.;
     sX = 1.;
     if (z != 0.) {
       const double ih = rsqrt64(h2);
-      cX = a * ih;
-      sX = az * ih;
+      cX = fabs(a) * ih;
+      sX = copysign(az, a) * ih;
     }
   } else {
     rp_X = fma(-az, J.cot_x, r);
