@@ -217,7 +217,9 @@ __device__ __forceinline__ void jf12_field(const Jf12Dev &J, double x, double y,
   // toroidal halo (:122-139)
   const bool north = z >= 0;
   const double b1 = north ? J.p.Bn : J.p.Bs, rh = north ? J.p.rn : J.p.rs;
-  const double B_h = b1 * logistic64(J.i2wh * (rh - r)) * exp64<true>(-az * J.iz0);
+  // 1 - step as in the reference: exactly 0 beyond the edge, where step(-x) would
+  // leave a field of e^-x whose square the FP32 loop cannot invert
+  const double B_h = b1 * (1. - logistic64(J.i2wh * (r - rh))) * exp64<true>(-az * J.iz0);
   cyl1 = fma(B_h, zprofile, cyl1);
   // X field (:141-170)
   const double rc_X = fma(az, J.cot_x, J.p.rpc_X);

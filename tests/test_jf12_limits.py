@@ -1,9 +1,9 @@
-"""Breg_jf12 over the X-field angles that the model takes: level (the radius that
-bounds the inner region is infinite off the plane), steep, and beyond a right
-angle or below zero, where the inner region's angle changes sign.  Faraday depth
-maps of an exponential disk against a plain numpy sum of the reference's
-expressions (breg_jf12.cc:72-186): 1e-10 of the map maximum in FP64 (the parity
-suite's bar), 1e-5 in FP32C."""
+"""Breg_jf12 at its limits.  Over the X-field angles that the model takes: level
+(the radius that bounds the inner region is infinite off the plane), steep, and
+beyond a right angle or below zero, where the inner region's angle changes sign.
+Faraday depth maps of an exponential disk against a plain numpy sum of the
+reference's expressions (breg_jf12.cc:72-186): 1e-10 of the map maximum in FP64
+(the parity suite's bar), 1e-5 in FP32C."""
 import math
 
 import numpy as np
@@ -92,3 +92,23 @@ def test_faraday_depth_vs_numpy(oracle, form, tol, angle):
             got = ig.write_grid(o)["fd"]
         assert np.isfinite(got).all()
         assert rel_err(got, _fd(oracle, o, angle)) <= tol, observer
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("alpha", [1.0, 2.7, 3.0])
+def test_beyond_the_halo_edge(alpha):
+    """Without an X field nothing is left some wh beyond the halo's edge: the sky
+    there is empty and finite, and both forms agree (1e-5, the FP32C bar)."""
+    from hammurabix_b200.integrator import Integrator
+    m = _models(49.0)
+    m.jf12.B0_X = 0.0
+    m.cre_ana.alpha = alpha
+    o = W.make_obs([8], 24.0, 0.05, freq_ghz=23.0, observer_kpc=(-16.0, 0.0, 3.0))
+    got = {}
+    for form in ("fp64", "fp32c"):
+        with Integrator(form) as ig:
+            ig.set_models(m)
+            got[form] = ig.write_grid(o)
+    for k, a in got["fp64"].items():
+        assert np.isfinite(a).all() and np.abs(a).max() > 0 and a.min() > -1e20, k
+        assert rel_err(got["fp32c"][k], a) <= 1e-5, k
