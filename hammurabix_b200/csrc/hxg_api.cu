@@ -1860,6 +1860,30 @@ int fused_shell(hxg_handle *h, const hxg_obs_t *o, uint32_t s, uint32_t shard, u
   return HXG_OK;
 }
 
+// Whether passes o[0..n) may write their maps m[5 k + j] (map j of pass k) side by
+// side: no memory in common but whole DM or FD maps, which are the same for every
+// pass.  Others must be written in turn, the last pass's values staying.
+bool outputs_apart(const hxg_obs_t *o, int n, double *const *m) {
+  struct Map {
+    uintptr_t at, end;
+    int kind;
+  };
+  std::vector<Map> all;
+  for (int k = 0; k < n; ++k)
+    for (int j = 0; j < 5; ++j) {
+      if (!(j == 0 ? o[k].do_dm : j == 1 ? o[k].do_fd : o[k].do_sync)) continue;
+      const uint32_t ns = j == 0 ? o[k].nside_dm : j == 1 ? o[k].nside_fd : o[k].nside_sync;
+      const uintptr_t at = reinterpret_cast<uintptr_t>(m[5 * k + j]);
+      const Map x{at, at + npix_of(ns) * sizeof(double), j};
+      for (const Map &y : all) {
+        const bool same = x.at == y.at && x.end == y.end && x.kind == y.kind && j < 2;
+        if (!same && x.at < y.end && y.at < x.end) return false;
+      }
+      all.push_back(x);
+    }
+  return true;
+}
+
 // nf (2 or 3) fusable passes in one traversal per shell; outs[5 k + j] =
 // map j (dm, fd, is, qs, us) of pass k.
 template <int NF>
@@ -1877,7 +1901,13 @@ int write_fused(hxg_handle *h, const hxg_obs_t *o, double *const *outs) {
   double *base[HXG_MAX_SHELLS];
   if ((st = shell_blocks(h, o0, 1 + 3 * NF, base)) != HXG_OK) return st;
   // the pass outputs start at zero (hxg_write_grid_device); the inner-shell FD
-  // is read from the first pass that accumulates FD
+  // is read from the first pass that accumulates FD; a DM or FD map that several
+  // passes share is written once
+  const auto first_use = [&](int f, int j) {
+    for (int c = 0; c < f; ++c)
+      if ((j == 0 ? o[c].do_dm : o[c].do_fd) && outs[5 * c + j] == outs[5 * f + j]) return false;
+    return true;
+  };
   bool any_fd = false;
   int fd_pass = -1;
   for (int f = 0; f < NF; ++f) {
@@ -1904,9 +1934,10 @@ int write_fused(hxg_handle *h, const hxg_obs_t *o, double *const *outs) {
       std::vector<const double *> sr;
       for (int c = a; c < NF; ++c)
         if (o[c].do_fd && !done[c] && o[c].nside_fd == o[a].nside_fd) {
+          done[c] = true;
+          if (!first_use(c, 1)) continue;
           d.push_back(outs[5 * c + 1]);
           sr.push_back(tmp_fd);
-          done[c] = true;
         }
       InterpTab tab;
       if ((st = interp_tab(h, o[a].nside_fd, o0.nside_shell[s], &tab)) != HXG_OK) return st;
@@ -1918,7 +1949,7 @@ int write_fused(hxg_handle *h, const hxg_obs_t *o, double *const *outs) {
   std::vector<PassOut> pouts;
   for (int f = 0; f < NF; ++f) {
     double *const *m = outs + 5 * f;
-    if (o[f].do_dm) pouts.push_back({o[f].nside_dm, 0, m[0]});
+    if (o[f].do_dm && first_use(f, 0)) pouts.push_back({o[f].nside_dm, 0, m[0]});
     for (int j = 0; j < 3; ++j) pouts.push_back({o[f].nside_sync, 1 + 3 * f + j, m[2 + j]});
   }
   if ((st = merge_pass(h, o0, base, pouts)) != HXG_OK) return st;
@@ -1942,7 +1973,9 @@ int hxg_write_grid_multi(hxg_handle *h, int npass, const hxg_obs_t *obs, double 
   int k = 0;
   while (k < npass) {
     const int left = npass - k;
-    const int nf = left >= 3 && fusable(h, obs + k, 3) ? 3 : (left >= 2 && fusable(h, obs + k, 2) ? 2 : 1);
+    int nf = 1;
+    for (int n = std::min(left, 3); n > 1 && nf == 1; --n)
+      if (fusable(h, obs + k, n) && outputs_apart(obs + k, n, d_outs + 5 * k)) nf = n;
     const auto one = [&](int q) {
       double *const *m = d_outs + 5 * q;
       return hxg_write_grid_device(h, obs + q, m[0], m[1], m[2], m[3], m[4]);

@@ -325,8 +325,10 @@ int hxg_sync(hxg_handle *h);
  * hxg_write_grid_device gives for that pass alone, to the form's rounding.
  * Other passes run one by one, and in the FP64 form also those of a handle
  * with checkpointing on (the adjoint then has the last pass's checkpoint) and
- * those whose shell maps do not fit the device together.  Asynchronous on
- * the handle's stream.  No counterpart in the reference.                   */
+ * those whose shell maps do not fit the device together.  Passes may share a
+ * DM or FD map; passes that share other output memory run one by one, so that
+ * the last one's values stay.  Asynchronous on the handle's stream.  No
+ * counterpart in the reference.                                             */
 int hxg_write_grid_multi(hxg_handle *h, int npass, const hxg_obs_t *obs,
                          double *const *d_outs);
 /* Same with host output buffers (outs[5k..5k+4] of pass k, NULL where the
