@@ -239,7 +239,7 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
           const double xv = bY, yv = fma(ct, bX, -(st * bz));
           const double x2 = xv * xv;
           const double rr = fma(yv, yv, x2), cc2 = fma(-yv, yv, x2), hs2 = xv * yv;
-          const double irr = rr > 1e-300 ? rcp64(rr) : 0.;
+          const double irr = rcp64(rr);
           double wt, wpc, wps, pe = P.em_pe;
           const double prof = (kFast || M.cre == kCreAna)
                                   ? cre_ana_prof64<!kFast>(F, r, az)
@@ -265,8 +265,10 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
               wp = base * gpp;
               pe = 1. - e;
             }
-            wpc = rr > 0. ? wp * (cc2 * irr) : wp;
-            wps = 2. * wp * (hs2 * irr);
+            double c2 = cc2 * irr, s2 = 2. * hs2 * irr;
+            if (rr < kTinyB2) angle64(xv, yv, c2, s2);
+            wpc = wp * c2;
+            wps = wp * s2;
           }
           double sf, cf;
           sincos_quarter(fma(P.quarter_k, sfd, q0), sf, cf);
@@ -279,6 +281,13 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
           const double ke = ej * pe * irr, ki = 2. * dG * irr;
           g_th = fma(ke, yv, ki * xv);
           g_ph = fma(ke, xv, -(ki * yv));
+          if (rr < kTinyB2) {  // both fields scaled, as in angle64
+            const double xs = xv * kTinyScale, ys = yv * kTinyScale;
+            const double ra = fma(ys, ys, xs * xs);
+            const double ira = ra > 0. ? kTinyScale * rcp64(ra) : 0.;
+            g_th = fma(ej * pe, ys, 2. * dG * xs) * ira;
+            g_ph = fma(ej * pe, xs, -(2. * dG * ys)) * ira;
+          }
         }
         g_te = fma(gk, bpar, g_te);
         g_bpar = gk * te;

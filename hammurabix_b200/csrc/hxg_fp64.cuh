@@ -224,6 +224,23 @@ __device__ __forceinline__ double bperp_pow64(const ShellLaunch &P, double b2) {
   return exp64<true>(0.5 * P.em_pe * log(b2));
 }
 
+// |B_perp|^2 in G^2 up to which the sums of squares lose their last bits or all of
+// them (a thin disk far from the plane): the angle then comes from fields scaled
+// by kTinyScale.
+constexpr double kTinyB2 = 1e-290;
+constexpr double kTinyScale = 0x1p500;
+
+// cos 2ipa and sin 2ipa of sky components (xv, yv) below that; ipa of a zero B_perp
+// is 0 (atan2(0, 0)).
+__device__ __forceinline__ void angle64(double xv, double yv, double &c2, double &s2) {
+  xv *= kTinyScale;
+  yv *= kTinyScale;
+  const double rr = fma(yv, yv, xv * xv);
+  const double inv = rr > 0. ? rcp64(rr) : 0.;
+  c2 = rr > 0. ? fma(-yv, yv, xv * xv) * inv : 1.;
+  s2 = 2. * (xv * yv) * inv;
+}
+
 // Warp gw of shell launch P (32/C pixels, C lanes each) for the NF frequency
 // passes of Fq.  All 32 lanes of the warp call it with the same gw.  kFast:
 // the launch's models satisfy fast_models and fast_ok (the other models and the
@@ -394,13 +411,14 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
                 wp[f] = base * gp;
               }
             }
-            // ipa of a zero B_perp is 0 (atan2(0, 0)): cos 2ipa = 1
-            const double inv = rr > 0. ? rcp64(rr) : 0.;
+            const double inv = rcp64(rr);
+            double c2 = cc2 * inv, s2 = 2. * hs2 * inv;
+            if (rr < kTinyB2) angle64(xv, yv, c2, s2);
 #pragma unroll
             for (int f = 0; f < NW; ++f) {
               if (f > 0 && shared_w) break;
-              wpc[f] = rr > 0. ? wp[f] * (cc2 * inv) : wp[f];
-              wps[f] = 2. * wp[f] * (hs2 * inv);
+              wpc[f] = wp[f] * c2;
+              wps[f] = wp[f] * s2;
             }
           }
         }
