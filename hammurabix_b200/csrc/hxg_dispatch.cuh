@@ -3,9 +3,21 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <type_traits>
 
 namespace hxg {
+
+// The grid-group count by whose instantiation an FP64 launch runs.  The one-grid
+// kernels read a voxel record in one 32-byte load and index records with 32 bits;
+// a caller's own records (hxg_write_grid_noalloc) need only 16-byte alignment and
+// can be more than 2^32 - 1, so those take the kernel for several grids, whose
+// loads are 16 bytes wide and whose indices have 64 bits.
+inline int fp64_groups(int ngroups, const void *rec, int nx, int ny, int nz) {
+  const bool one = (reinterpret_cast<uintptr_t>(rec) & 31) == 0 &&
+                   (unsigned __int128)nx * ny * nz <= 0xFFFFFFFFu;
+  return ngroups == 1 && !one ? 2 : ngroups;
+}
 
 // The kernels are instantiated per grid-group count (0, 1, up to
 // kMaxGroups) and per use of the Jaffe / JF12 / YMW16 blocks.

@@ -5,12 +5,9 @@
 
 namespace hxg {
 
-// The one-grid kernels read 32-byte records in one load.  Records that the
-// caller packed (hxg_write_grid_noalloc) need be aligned to 16 bytes only;
-// those take the kernel for several grids, whose loads are 16 bytes wide.
 static int shape64(const ShellLaunch &P) {
-  const bool wide = P.ngroups != 1 || (reinterpret_cast<uintptr_t>(P.groups[0].rec) & 31) == 0;
-  return wide ? P.ngroups : kMaxGroups;
+  const DevGridGroup &G = P.groups[0];
+  return fp64_groups(P.ngroups, G.rec, G.nx, G.ny, G.nz);
 }
 
 cudaError_t launch_shell64(cudaStream_t s, const ShellLaunch &P, unsigned blocks,

@@ -138,8 +138,8 @@ __device__ __forceinline__ void load_rec32(const double2 *p, double2 &a, double2
       : "l"(p));
 }
 
-// The cell of a sample: record index of its corner 000 (32 bits: the host
-// refuses larger grids), the (x, y) weights and the z weights.
+// The cell of a sample: record index of its corner 000 (32 bits: larger grids take
+// the kernel for several grids, fp64_groups), the (x, y) weights and the z weights.
 struct Cell64 {
   unsigned key;
   double w4[4], ez, fz;
