@@ -225,10 +225,14 @@ __device__ __forceinline__ void jf12_field(const Jf12Dev &J, double x, double y,
   const double rc_X = fma(az, J.cot_x, J.p.rpc_X);
   double rp_X, B_X, cX = J.cos_x, sX = J.sin_x;
   if (r < rc_X) {
-    // a division as in the reference: rc_X is infinite for Xtheta = 0, and near
-    // the plane r - rp_X is all cancellation
-    rp_X = r * J.p.rpc_X / rc_X;
-    const double q = rp_X * ir;
+    double q = J.p.rpc_X * rcp64(rc_X);
+    rp_X = r * q;
+    // rc_X is infinite for Xtheta = 0, and within the rounding of rpc_X r - rp_X is
+    // all cancellation: there the reference's quotients
+    if (!(fabs(rc_X - J.p.rpc_X) > 1e-9 * fabs(J.p.rpc_X)) || rc_X > 1e300) {
+      rp_X = r * J.p.rpc_X / rc_X;
+      q = J.p.rpc_X / rc_X;
+    }
     B_X = q * q;
     // cos and sin of atan(|z| / (r - rp_X)), which is negative where rp_X is
     // beyond r (rc_X below rpc_X); a right angle in the plane
