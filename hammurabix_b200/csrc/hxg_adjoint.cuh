@@ -284,9 +284,9 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
           if (rr < kTinyB2) {  // both fields scaled, as in angle64
             const double xs = xv * kTinyScale, ys = yv * kTinyScale;
             const double ra = fma(ys, ys, xs * xs);
-            const double ira = ra > 0. ? kTinyScale * rcp64(ra) : 0.;
-            g_th = fma(ej * pe, ys, 2. * dG * xs) * ira;
-            g_ph = fma(ej * pe, xs, -(2. * dG * ys)) * ira;
+            const double ira = ra > kTinyB2 ? rcp64(ra) : 0.;
+            g_th = fma(ej * pe, ys, 2. * dG * xs) * ira * kTinyScale;
+            g_ph = fma(ej * pe, xs, -(2. * dG * ys)) * ira * kTinyScale;
           }
         }
         g_te = fma(gk, bpar, g_te);

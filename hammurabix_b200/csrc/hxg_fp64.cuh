@@ -231,13 +231,13 @@ constexpr double kTinyB2 = 1e-290;
 constexpr double kTinyScale = 0x1p500;
 
 // cos 2ipa and sin 2ipa of sky components (xv, yv) below that; ipa of a zero B_perp
-// is 0 (atan2(0, 0)).
+// is 0 (atan2(0, 0)), and so is that of one below 1e-295 G.
 __device__ __forceinline__ void angle64(double xv, double yv, double &c2, double &s2) {
   xv *= kTinyScale;
   yv *= kTinyScale;
   const double rr = fma(yv, yv, xv * xv);
-  const double inv = rr > 0. ? rcp64(rr) : 0.;
-  c2 = rr > 0. ? fma(-yv, yv, xv * xv) * inv : 1.;
+  const double inv = rr > kTinyB2 ? rcp64(rr) : 0.;
+  c2 = rr > kTinyB2 ? fma(-yv, yv, xv * xv) * inv : 1.;
   s2 = 2. * (xv * yv) * inv;
 }
 

@@ -67,3 +67,12 @@ def test_scaled_field(alpha, power, tol):
         if abs(par[k]) / f < 1e-290:
             continue                # the scaled gradient is no normal number
         assert abs(tpar[k] * f - par[k]) <= tol * abs(par[k]), k
+
+
+@pytest.mark.parametrize("alpha", [2.7, 3.0])
+@pytest.mark.parametrize("power", [-960, -1000, -1020, -1040])
+def test_fields_near_the_smallest_number(alpha, power):
+    """Fields of 1e-294 to 1e-318 G: no emission and no gradient, and no NaN."""
+    maps, par = _run(2.0 ** power, alpha)
+    assert all((t == 0).all() for t in maps)
+    assert np.isfinite(par).all()
