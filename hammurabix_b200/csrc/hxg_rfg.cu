@@ -76,26 +76,6 @@ __device__ inline double kcomp(int i, int n, double L) {
   return k;
 }
 
-// x^a for normal x > 0 to about one ulp: x = 2^E m with m in [0.7, 1.42), and
-// a E split into an integer and a rest, so that the argument of the one
-// exponential stays below about |a| / 2 and its rounding with it.
-__device__ inline double pow_k(double x, double a) {
-  int hi = __double2hiint(x);
-  const int e = ((hi - 0x3fe6a09e) >> 20);
-  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
-  const double E = (double)e, p = a * E;
-  if (!(fabs(p) < 900.) || hi < 0x00100000 || hi >= 0x7ff00000) return pow(x, a);
-  const double n = rint(p);
-  const double r = fma((p - n) + fma(a, E, -p), 0.6931471805599453, a * log(m));
-  return ldexp(exp64<true>(r), (int)n);
-}
-
-// sqrt of v >= 0
-__device__ inline double sqrt_pos(double v) {
-  double ir;
-  return v > 1e-290 ? sqrt64(v, ir) : sqrt(v);
-}
-
 // TErnd_dft::spectrum (ternd_dft.cc:17-24)
 __device__ inline double spec_dft(double k, const hxg_ternd_dft_t &p) {
   if (k < p.k0) return 0.;
