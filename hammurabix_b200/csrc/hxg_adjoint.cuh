@@ -149,10 +149,6 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     const DevModels &M = P.models;
     const FastModels &F = P.fast;
     const double oz = P.obs[2];
-    const double oX = fma(cp, P.obs[0], sp * P.obs[1]);
-    const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
-    const double YY = fma(Y, Y, 1e-280);
-    const double csY = F.sp_cos * Y, ssY = F.sp_sin * Y;
     const bool fast_b = M.breg == kBregSpiral;
     const bool fast_t = M.tereg == kTeregExpdisk;
     const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
@@ -180,6 +176,8 @@ shell_fp64_adjoint_kernel(const AdjointLaunch A) {
     chunk_range64(P, u, c, i0, i1);
     int ga = i1, gb = i1;
     if (NG == 1) grid_range64(P, P.groups[0], u, i0, i1, ga, gb);
+    double oX, YY, csY, ssY;
+    turned_observer(P, st, cp, sp, i0, i1, oX, YY, csY, ssY);
     double x = (double)i0 + 0.5;
 #pragma unroll 1
     for (int i = i0; i < i1; ++i, x += 1.) {

@@ -88,6 +88,26 @@ __device__ __forceinline__ void chunk_range64(const ShellLaunch &P, const double
   i1 = (int)(lo + ((n * (c + 1)) >> P.log2_chunks));
 }
 
+// The observer in the frame turned by the ray's azimuth, (oX, Y): r^2 along the ray
+// is X^2 + YY with X = st d + oX, never 0, so that 1/r is finite; csY and ssY are Y
+// times the cos and sin of the spiral's pitch.  Rounding of oX and Y moves every
+// sample of the ray alike, so their second parts go into the constants: into csY, ssY
+// and Y^2 exactly, 2 X oXl into YY with the X of the middle of the samples [i0, i1).
+// Error of Q, U at 1.4 GHz against an extended-precision integral (Nside 4/8/16, 32^3
+// grids, mean of 24 skies): 4.4e-15, 4.5e-15 without, 3.8e-15, 4.2e-15 with.
+__device__ __forceinline__ void turned_observer(const ShellLaunch &P, double st, double cp,
+                                                double sp, int i0, int i1, double &oX,
+                                                double &YY, double &csY, double &ssY) {
+  const FastModels &F = P.fast;
+  double oXl, Y, Yl;
+  dot2_64(cp, P.obs[0], sp, P.obs[1], oX, oXl);
+  dot2_64(cp, P.obs[1], -sp, P.obs[0], Y, Yl);
+  const double Xm = fma(st, fma(0.5 * ((double)i0 + (double)i1), P.delta, P.d_start), oX);
+  YY = fmax(fma(Y, Y, 2. * fma(Y, Yl, Xm * oXl)), 1e-280);
+  csY = fma(F.sp_cos, Y, fma(F.sp_cos, Yl, -(F.sp_sin * oXl)));
+  ssY = fma(F.sp_sin, Y, fma(F.sp_sin, Yl, F.sp_cos * oXl));
+}
+
 // Grid coordinate k of the ray at distance d: (observer - lo + u d) scale, the
 // rounding of observer - lo, which would move every sample of every ray the
 // same way, added back.
@@ -282,12 +302,6 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
     const DevModels &M = P.models;
     const FastModels &F = P.fast;
     const double oz = P.obs[2];
-    // the observer in the frame turned by the ray's azimuth
-    const double oX = fma(cp, P.obs[0], sp * P.obs[1]);
-    const double Y = fma(cp, P.obs[1], -(sp * P.obs[0]));
-    // r^2 along the ray is X^2 + YY; never 0, so that 1/r is finite
-    const double YY = fma(Y, Y, 1e-280);
-    const double csY = F.sp_cos * Y, ssY = F.sp_sin * Y;
     const bool fast_b = M.breg == kBregSpiral;
     const bool fast_t = M.tereg == kTeregExpdisk;
     const bool slow_b = !kFast && M.breg != kBregNone && !fast_b;
@@ -304,6 +318,8 @@ __device__ __forceinline__ void fp64_tile(const ShellLaunch &P, const FreqSet<NF
     chunk_range64(P, u, c, i0, i1);
     int ga = i1, gb = i1;
     if (NG == 1) grid_range64(P, P.groups[0], u, i0, i1, ga, gb);
+    double oX, YY, csY, ssY;
+    turned_observer(P, st, cp, sp, i0, i1, oX, YY, csY, ssY);
     double x = (double)i0 + 0.5;
 #pragma unroll 1
     for (int i = i0; i < i1; ++i, x += 1.) {

@@ -137,6 +137,16 @@ __device__ __forceinline__ void sincos_quarter(double h, double &s, double &c) {
   c = __hiloint2double(__double2hiint(b) ^ (((n + 1) & 2) << 30), __double2loint(b));
 }
 
+// a b + c d in two parts, to 4 u^2 (|a b| + |c d|): the products' and the sum's rounding
+// errors are exact (FMA; Knuth's two-sum).
+__device__ __forceinline__ void dot2_64(double a, double b, double c, double d, double &hi,
+                                        double &lo) {
+  const double p = a * b, q = c * d;
+  hi = p + q;
+  const double t = hi - p;
+  lo = ((p - (hi - t)) + (q - t)) + (fma(a, b, -p) + fma(c, d, -q));
+}
+
 // x^a for normal x > 0: x = 2^E m with m in [0.7, 1.42), and a E split into an integer
 // and a rest, so that the argument of the one exponential stays below about |a| / 2 and
 // its rounding with it.  Within (1.5 |a| + 4) u relative: 1.1 |a| u of a log m, 0.4 |a| u

@@ -15,6 +15,7 @@ __global__ void eval(int f, int n, const double *a, const double *b, double *out
     case 4: r = hxg::rcp64(x); break;
     case 5: hxg::sincos_quarter(x, r, s); break;
     case 6: r = hxg::pow_k(x, b[i]); break;
+    case 8: hxg::dot2_64(x, b[i], a[n - 1 - i], b[n - 1 - i], r, s); break;
     case 7: r = hxg::sqrt_pos(x); break;
   }
   out[i] = r;

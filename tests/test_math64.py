@@ -6,6 +6,7 @@ import ctypes as C
 import os
 import shutil
 import subprocess
+from fractions import Fraction as F
 
 import numpy as np
 import pytest
@@ -18,7 +19,7 @@ CSRC = os.path.join(os.path.dirname(HERE), "hammurabix_b200", "csrc")
 L = np.longdouble
 PI = L("3.14159265358979323846264338327950288")
 U = 2.0 ** -53
-EXP, EXP_IN, RSQRT, SQRT, RCP, SINCOS, POW, SQRT_POS = range(8)
+EXP, EXP_IN, RSQRT, SQRT, RCP, SINCOS, POW, SQRT_POS, DOT2 = range(9)
 
 
 @pytest.fixture(scope="module")
@@ -154,3 +155,14 @@ def test_pow_k_outside_its_range(fn):
         want = np.power(x, a)
     assert np.isnan(got[4]) and np.allclose(np.delete(got, 4), np.delete(want, 4), rtol=1e-14,
                                             atol=0)
+
+
+def test_dot2_64(fn):
+    """a b + c d of pairs from both ends of the arrays, exact in rationals."""
+    r = _rng()
+    a, b = r.uniform(-1, 1, 3000), r.uniform(-1, 1, 3000) * 2.5e22
+    a[:500], b[:500] = np.cos(r.uniform(0, 6.3, 500)), -2.561e22
+    hi, lo = fn(DOT2, a, b)
+    for k in range(len(a)):
+        x, y = F(a[k]) * F(b[k]), F(a[-1 - k]) * F(b[-1 - k])
+        assert abs(F(hi[k]) + F(lo[k]) - (x + y)) <= F(4 * U * U) * (abs(x) + abs(y)), k
