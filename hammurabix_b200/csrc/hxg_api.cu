@@ -2719,6 +2719,7 @@ struct hxg_batch {
   bool fp32 = false;
   int ngroups = 0;
   int lanes = 1, grain = 4, tried = 0;
+  std::vector<int> shape;   // lanes of every plan, and the grain where it matters
   double best_ms = 0.;
   int64_t samples = 0;
   std::vector<size_t> tmp_off;  // per entry, doubles into tmp
@@ -2767,25 +2768,38 @@ int upload_vec(hxg_handle *h, DevBuf &b, const std::vector<T> &v) {
   return HXG_OK;
 }
 
-// A batch level's plans get a kernel each, run side by side in the graph, with
-// the launch block in constant memory and the launch shape of the single
-// pass; the persistent kernel, which reads its plans from global memory at 16
-// warps per SM, is left the FP32C plans of under kSmallTiles warp tiles where
-// a level has more than kManyPlans of them: there the kernels' count (128 run
-// at a time) takes longer than the work.  Measured (ms, persistent / one
-// kernel each): 16 sets x 3 frequencies, Nside 64/128/256 95.8 / 73.1; 24 sets,
-// Nside 16 5.42 / 1.48; 200 sets, Nside 8 2.44 / 1.51; 600 sets, Nside 4/8
-// 2.83 / 3.70.
+// How a batch level's plans are launched.  A plan of kOwnBlocks blocks and more gets a
+// kernel of its own, smaller ones go kGroupPlans to a kernel; both have the launch
+// blocks in constant memory and the launch shape of the single pass, and run side by
+// side in the graph.  The persistent kernel, which reads its plans from global memory at
+// 16 warps per SM, is left the FP32C plans of under kSmallTiles warp tiles where a level
+// has more than kManyPlans of them (600 sets of Nside 4/8 1.46 ms a run, 1.67 in
+// groups).  Instantiating the graph costs 50 us for each parallel kernel and 8 us for
+// one behind another, so own kernels take as many chains as fill the device eight times,
+// kMinChains to kMaxChains, groups half of kMaxChains.  A kernel's plans are read by
+// index: a large plan is 8-11 % slower in a group than alone.
+// hxg_batch_create + run in ms, by (a) the persistent kernel with FP64 passes unfused,
+// (b) every plan in a chain of its own, up to 128, (c) now:
+//   FP32C 16 sets x 3 frequencies, Nside 64/128/256  4.5 + 95.2   4.5 + 72.7   2.8 + 72.7
+//         64 sets, Nside 8/16/32                     1.0 + 2.9   11.3 + 1.7    2.3 + 2.1
+//         200 sets x 3, Nside 8                      2.4 + 1.1    9.6 + 0.7    2.9 + 0.7
+//   FP64  16 sets x 2, Nside 32/64                   1.1 + 30.1   2.8 + 5.2    1.9 + 5.2
+//         64 sets, Nside 8/16/32                     1.0 + 8.1   11.5 + 2.1    2.7 + 2.2
+//         200 sets x 3, Nside 8                      2.4 + 5.0   10.3 + 1.0    3.0 + 1.0
+//         600 sets, Nside 4/8                        2.6 + 3.9   18.9 + 2.2    6.0 + 1.8
+//         2000 sets x 2, Nside 2/4                  16.6 + 5.8   49.0 + 4.1   26.8 + 2.6
+constexpr unsigned kOwnBlocks = 64;
 constexpr unsigned long long kSmallTiles = 64;
-constexpr size_t kManyPlans = 256;
+constexpr size_t kManyPlans = 256, kMinChains = 4, kMaxChains = 16;
 
 // Device tables of a batch for one launch shape.
 int batch_tables(hxg_batch *b, int lanes, int grain) {
   hxg_handle *h = b->h;
   int st;
-  b->lanes = lanes;
-  b->grain = grain;
+  b->grain = 0;
   b->samples = 0;
+  b->shape.clear();
+  unsigned long long most = 0;  // work of the plan whose lanes are reported
   double *tmp = static_cast<double *>(b->tmp.p);
   const auto map = [&](size_t i, int k) { return tmp + b->tmp_off[i] + k * b->tmp_n[i]; };
   for (int s = 0; s < b->levels; ++s) {
@@ -2797,15 +2811,28 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
     std::vector<MergeJob> mj;
     std::vector<unsigned long long> m0(1, 0ull);
     b->direct[s].clear();
-    // pixels of the level, and its plans too small for a kernel of their own
+    // pixels of the level, and its plans of few warp tiles
     uint64_t level_pix = 0;
     size_t small = 0;
-    for (size_t i = 0; i < b->e.size(); i += (size_t)b->group[i]) {
-      const hxg_obs_t &o = b->e[i].obs;
-      if ((uint32_t)s >= o.total_shell) continue;
-      level_pix += npix_of(o.nside_shell[s]);
-      small += npix_of(o.nside_shell[s]) * (uint64_t)lanes < 32 * kSmallTiles;
-    }
+    const auto of_level = [&](size_t i) { return (uint32_t)s < b->e[i].obs.total_shell; };
+    for (size_t i = 0; i < b->e.size(); i += (size_t)b->group[i])
+      if (of_level(i)) level_pix += npix_of(b->e[i].obs.nside_shell[s]);
+    const auto lanes_of = [&](const hxg_obs_t &o) {
+      double d0, dl;
+      uint64_t step;
+      shell_ref(o, (uint32_t)s, d0, dl, step);
+      int C = std::min(lanes, 32);
+      // the FP64 form cuts a ray's own window, so more lanes cost it little:
+      // enough of them for the level's plans to fill the device
+      if (!b->fp32) C = std::max(C, choose_chunks(h, level_pix, step));
+      while (C > 1 && step / (uint64_t)C < 16) C >>= 1;
+      return C;
+    };
+    const auto tiles_of = [&](const hxg_obs_t &o, int C) {
+      return (unsigned long long)(npix_of(o.nside_shell[s]) * (uint64_t)C + 31) / 32;
+    };
+    for (size_t i = 0; i < b->e.size(); i += (size_t)b->group[i])
+      if (of_level(i)) small += tiles_of(b->e[i].obs, lanes_of(b->e[i].obs)) < kSmallTiles;
     int tab_st = HXG_OK;
     const auto job = [&](int nmaps, double *const *d, const double *const *src, uint32_t nd,
                          int ns) {
@@ -2826,7 +2853,7 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
       const int nf = b->group[i];
       const hxg_batch_entry_t &E = b->e[i];
       const hxg_obs_t &o = E.obs;
-      if ((uint32_t)s >= o.total_shell) continue;
+      if (!of_level(i)) continue;
       ShellLaunch L;
       uint64_t step;
       if ((st = build_launch(h, E.models, o, (uint32_t)s, L, step)) != HXG_OK) return st;
@@ -2834,16 +2861,18 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
       L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) + i : nullptr;
       // an FP32C batch runs all its plans in one instantiation
       if (b->fp32 && !b->fast) L.fast_ok = 0;
-      int C = std::min(lanes, 32);
-      // the FP64 form cuts a ray's own window, so more lanes cost it little:
-      // enough of them for the level's plans to fill the device
-      if (!b->fp32) C = std::max(C, choose_chunks(h, level_pix, step));
-      while (C > 1 && step / (uint64_t)C < 16) C >>= 1;
+      const int C = lanes_of(o);
       L.chunks = C;
       L.log2_chunks = hxg::hpx_ilog2((uint64_t)C);
       const uint64_t npix = npix_of(o.nside_shell[s]);
       const int ns = (int)o.nside_shell[s];
-      const unsigned long long tiles = (npix * C + 31) / 32;
+      const unsigned long long tiles = tiles_of(o, C);
+      const unsigned long long work = tiles * (step / (uint64_t)C);
+      b->shape.push_back(C);
+      if (work > most) {
+        most = work;
+        b->lanes = C;
+      }
       b->samples += (int64_t)(npix * step * nf);
       // inner-shell FD and the shared DM / FD shell maps: the first pass of
       // the group that accumulates FD; DM / FD shell maps live in the
@@ -2868,9 +2897,11 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
       }
       const auto freqs = [&](auto &F) -> int {
         for (int f = 0; f < nf; ++f) {
-          ShellLaunch Lf;
+          ShellLaunch Lf = L;  // its constants are the first pass's
           uint64_t sf;
-          const int r = build_launch(h, b->e[i + f].models, b->e[i + f].obs, (uint32_t)s, Lf, sf);
+          const int r = f == 0 ? (int)HXG_OK
+                               : build_launch(h, b->e[i + f].models, b->e[i + f].obs, (uint32_t)s,
+                                              Lf, sf);
           if (r != HXG_OK) return r;
           F.lambda2[f] = Lf.lambda2;
           F.phase_k[f] = Lf.phase_k;
@@ -2891,7 +2922,7 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
         PlanLaunch D{};
         D.nf = nf;
         D.tiles = tiles;
-        D.work = tiles * (step / (uint64_t)C);
+        D.work = work;
         D.P = L;
         if (nf == 2 && (st = freqs(D.F2)) != HXG_OK) return st;
         if (nf == 3 && (st = freqs(D.F3)) != HXG_OK) return st;
@@ -2909,7 +2940,10 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
         if ((st = freqs(FP.F)) != HXG_OK) return st;
         P3.push_back(FP);
       }
-      if (!alone) t0[nf - 1].push_back(t0[nf - 1].back() + tiles);
+      if (!alone) {
+        t0[nf - 1].push_back(t0[nf - 1].back() + tiles);
+        b->grain = grain;
+      }
       for (int f = 0; f < nf; ++f) {
         const hxg_batch_entry_t &Ef = b->e[i + f];
         const hxg_obs_t &of = Ef.obs;
@@ -2945,27 +2979,88 @@ int batch_tables(hxg_batch *b, int lanes, int grain) {
     if ((st = upload_vec(h, b->merges[s], mj)) != HXG_OK) return st;
     if ((st = upload_vec(h, b->mblocks[s], m0)) != HXG_OK) return st;
   }
+  b->shape.push_back(b->grain);
   return HXG_OK;
 }
 
-// The plans of a level with kernels of their own, side by side in the graph
-// that s is capturing: up to kChains chains of kernels (the device runs 128
-// kernels at a time), the heaviest plans first, each to the shortest chain.  A
-// chain's next kernel is captured on s with the chain's last kernel as its
-// dependency.
+// Plans of one instantiation, at most kGroupPlans, as one kernel on s.
+template <int NF>
+cudaError_t launch_group(hxg_batch *b, const std::vector<const PlanLaunch *> &plans,
+                         cudaStream_t s) {
+  static_assert(HXG_FP32C_THREADS == HXG_FP32C_MULTI_THREADS, "one group launch shape");
+  const unsigned threads = b->fp32 ? HXG_FP32C_THREADS : HXG_FP64_THREADS;
+  auto G = std::make_unique<hxg::PlanGroup<NF>>();
+  unsigned at = 0;
+  for (size_t k = 0; k < (size_t)hxg::kGroupPlans; ++k) {
+    const PlanLaunch &D = *plans[std::min(k, plans.size() - 1)];
+    if (k < plans.size()) at += (unsigned)((D.tiles * 32 + threads - 1) / threads);
+    G->end[k] = at;
+    if (k >= plans.size()) continue;
+    G->P[k] = D.P;
+    if constexpr (NF == 1)
+      hxg::freq_of_launch(D.P, G->F[k]);
+    else if constexpr (NF == 2)
+      G->F[k] = D.F2;
+    else
+      G->F[k] = D.F3;
+  }
+  return hxg::launch_shell_group(s, b->fp32, NF, G->P[0], G.get(), at, threads);
+}
+
+// The plans of a level that the persistent kernel does not take, in the graph that s
+// is capturing: chains of kernels side by side, the heaviest first, each to the
+// shortest chain.  A chain's next kernel is captured on s with the chain's last kernel
+// as its dependency.
 cudaError_t launch_direct(hxg_batch *b, std::vector<PlanLaunch> &plans, cudaStream_t s) {
-  constexpr size_t kChains = 128;
+  const unsigned threads = b->fp32 ? HXG_FP32C_THREADS : HXG_FP64_THREADS;
+  const auto blocks_of = [&](const PlanLaunch &D) {
+    return (unsigned)((D.tiles * 32 + threads - 1) / threads);
+  };
   std::stable_sort(plans.begin(), plans.end(),
                    [](const PlanLaunch &x, const PlanLaunch &y) { return x.work > y.work; });
+  // kernels: one plan of kOwnBlocks and more, or up to kGroupPlans of one instantiation
+  struct Kernel {
+    std::vector<const PlanLaunch *> plans;
+    unsigned long long work = 0;
+  };
+  std::vector<Kernel> kernels;
+  std::map<std::pair<int, int>, size_t> open;  // (passes, instantiation): group being filled
+  size_t own = 0;
+  unsigned long long own_blocks = 0;
+  for (const PlanLaunch &D : plans) {
+    if (blocks_of(D) >= kOwnBlocks) {
+      ++own;
+      own_blocks += blocks_of(D);
+      kernels.push_back({{&D}, D.work});
+      continue;
+    }
+    const auto key = std::make_pair(D.nf, hxg::shell_instance(b->fp32, D.P));
+    const auto it = open.find(key);
+    if (it == open.end() || kernels[it->second].plans.size() == (size_t)hxg::kGroupPlans) {
+      open[key] = kernels.size();
+      kernels.push_back({});
+    }
+    Kernel &K = kernels[open[key]];
+    K.plans.push_back(&D);
+    K.work += D.work;
+  }
+  size_t n = kMaxChains / 2;
+  if (own) {
+    const double resident = 5. * b->h->sm_count;  // blocks of the launch shape at a time
+    n = (size_t)std::ceil(8. * resident * (double)own / (double)own_blocks);
+    n = std::max(kMinChains, std::min(kMaxChains, n));
+    if (own < kernels.size()) n = std::max(n, kMaxChains / 2);
+  }
+  n = std::min(n, kernels.size());
   std::vector<cudaGraphNode_t> deps;
   const auto here = [&](std::vector<cudaGraphNode_t> &v) {
     cudaStreamCaptureStatus st;
     const cudaGraphNode_t *d = nullptr;
-    size_t n = 0;
-    const cudaError_t r = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &d, &n);
+    size_t nd = 0;
+    const cudaError_t r = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &d, &nd);
     if (r != cudaSuccess) return r;
     if (st != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
-    v.assign(d, d + n);
+    v.assign(d, d + nd);
     return cudaSuccess;
   };
   const auto from = [&](std::vector<cudaGraphNode_t> &v) {
@@ -2973,23 +3068,24 @@ cudaError_t launch_direct(hxg_batch *b, std::vector<PlanLaunch> &plans, cudaStre
                                                cudaStreamSetCaptureDependencies);
   };
   cudaError_t e = here(deps);
-  const size_t n = std::min(kChains, plans.size());
   std::vector<std::vector<cudaGraphNode_t>> tail(n, deps);
   std::vector<unsigned long long> load(n, 0ull);
-  for (const PlanLaunch &D : plans) {
+  for (const Kernel &K : kernels) {
     if (e != cudaSuccess) return e;
     const size_t k = std::min_element(load.begin(), load.end()) - load.begin();
-    load[k] += D.work;
+    load[k] += K.work;
     if ((e = from(tail[k])) != cudaSuccess) return e;
-    const unsigned threads =
-        !b->fp32 ? HXG_FP64_THREADS : (D.nf == 1 ? HXG_FP32C_THREADS : HXG_FP32C_MULTI_THREADS);
-    const unsigned blocks = (unsigned)((D.tiles * 32 + threads - 1) / threads);
-    if (D.nf == 1)
-      e = hxg::launch_shell(s, b->fp32, D.P, blocks, threads);
+    const PlanLaunch &D = *K.plans[0];
+    if (K.plans.size() > 1)
+      e = D.nf == 1   ? launch_group<1>(b, K.plans, s)
+          : D.nf == 2 ? launch_group<2>(b, K.plans, s)
+                      : launch_group<3>(b, K.plans, s);
+    else if (D.nf == 1)
+      e = hxg::launch_shell(s, b->fp32, D.P, blocks_of(D), threads);
     else
       e = hxg::launch_shell_multi(s, b->fp32, D.P, D.nf,
-                                  D.nf == 2 ? (const void *)&D.F2 : (const void *)&D.F3, blocks,
-                                  threads);
+                                  D.nf == 2 ? (const void *)&D.F2 : (const void *)&D.F3,
+                                  blocks_of(D), threads);
     ++b->graph_kernels;
     if (e == cudaSuccess) e = here(tail[k]);
   }
@@ -3221,13 +3317,18 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
     if (ce != cudaSuccess) return bail(cuda_fail(h, ce, "occupancy"));
     b->level_blocks[nf - 1] = (unsigned)std::max(1, per_sm) * (unsigned)h->sm_count;
   }
-  // launch shapes: lanes per pixel x tiles per work fetch
+  // launch shapes: lanes per pixel x tiles per work fetch; those that come to the same
+  // launches (a grain that no plan has, lanes that short rays do not take) once
   const int shapes[][2] = {{1, 4}, {2, 4}, {4, 4}, {8, 4}, {1, 16}, {2, 1}};
   int best = 0;
+  std::vector<std::vector<int>> timed;
+  std::vector<int> best_shape;
   if (tune) {
     double best_ms = 1e300;
     for (int k = 0; k < (int)(sizeof(shapes) / sizeof(shapes[0])); ++k) {
       if ((st = batch_tables(b, shapes[k][0], shapes[k][1])) != HXG_OK) return bail(st);
+      if (std::find(timed.begin(), timed.end(), b->shape) != timed.end()) continue;
+      timed.push_back(b->shape);
       if ((st = batch_capture(b)) != HXG_OK) return bail(st);
       double ms;
       if ((st = batch_time(b, &ms)) != HXG_OK) return bail(st);
@@ -3235,12 +3336,16 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
       if (ms < best_ms) {
         best_ms = ms;
         best = k;
+        best_shape = b->shape;
       }
     }
     b->best_ms = best_ms;
   }
-  if ((st = batch_tables(b, shapes[best][0], shapes[best][1])) != HXG_OK) return bail(st);
-  if ((st = batch_capture(b)) != HXG_OK) return bail(st);
+  // the graph of the best shape stays when it was the last one captured
+  if (timed.empty() || timed.back() != best_shape || b->shape != best_shape) {
+    if ((st = batch_tables(b, shapes[best][0], shapes[best][1])) != HXG_OK) return bail(st);
+    if ((st = batch_capture(b)) != HXG_OK) return bail(st);
+  }
   *out = b;
   return HXG_OK;
 }

@@ -1,9 +1,9 @@
 // hxg_batch.cuh -- batched forward: many independent passes (parameter
 // sets x frequencies) of Integrator::write_grid (integrator.cc:23-134) in
 // one CUDA graph.  Per shell level the graph holds the shell kernels of every
-// parameter set that has that shell, side by side (many small FP32C sets share
-// the persistent kernel below), and one kernel that merges the shell maps into
-// each entry's outputs (Hampix::accumulate, hamdis.h:698-721); the outer-shell
+// parameter set that has that shell, side by side (up to kGroupPlans small sets in
+// one; many small FP32C sets share the persistent kernel below), and one kernel that
+// merges the shell maps into each entry's outputs (Hampix::accumulate, hamdis.h:698-721); the outer-shell
 // levels read the inner Faraday depth the earlier levels accumulated
 // (integrator.cc:78-86).
 #pragma once

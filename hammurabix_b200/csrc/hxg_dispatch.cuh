@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -36,6 +37,22 @@ inline cudaError_t by_shape(int ngroups, bool ext, F &&f) {
   else
     g(std::integral_constant<int, 4>{});
   return cudaGetLastError();
+}
+
+// A number for the instantiation that by_shape and the kFast rule choose.
+inline int shell_key(int ngroups, bool ext, bool fast) {
+  return fast ? std::min(ngroups, 2) : 3 + 2 * std::min(ngroups, 2) + (ext ? 1 : 0);
+}
+
+// f with the pass count 1, 2 or 3 as a constant.
+template <typename F>
+inline void by_passes(int nf, F &&f) {
+  if (nf == 1)
+    f(std::integral_constant<int, 1>{});
+  else if (nf == 2)
+    f(std::integral_constant<int, 2>{});
+  else
+    f(std::integral_constant<int, 3>{});
 }
 
 }  // namespace hxg

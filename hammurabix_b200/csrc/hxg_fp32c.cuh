@@ -634,6 +634,19 @@ shell_fp32c_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
                            threadIdx.x & 31);
 }
 
+// The plans of a batch level, kGroupPlans to a kernel.
+template <int NG, bool kExt, int NF, bool kFast>
+__global__ void __launch_bounds__(HXG_FP32C_MULTI_THREADS,
+                                  kFast ? HXG_FP32C_MULTI_MIN_BLOCKS_FAST
+                                        : HXG_FP32C_MULTI_MIN_BLOCKS)
+shell_fp32c_group_kernel(const __grid_constant__ PlanGroup<NF> G) {
+  unsigned block;
+  const int k = group_plan(G, block);
+  fp32c_tile<NG, kExt, NF, kFast>(G.P[k], G.F[k],
+                                  ((long long)block * blockDim.x + threadIdx.x) >> 5,
+                                  threadIdx.x & 31);
+}
+
 // The second half of a launch whose lanes left their sums in P.part: the
 // chunk combination in the mapping, and so with the sums, of a launch that
 // keeps a pixel's chunks in one warp.

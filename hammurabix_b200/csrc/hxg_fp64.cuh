@@ -521,4 +521,16 @@ shell_fp64_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
                                  threadIdx.x & 31);
 }
 
+// The plans of a batch level, kGroupPlans to a kernel.
+template <int NG, bool kExt, int NF, bool kFast>
+__global__ void __launch_bounds__(HXG_FP64_THREADS,
+                                  kExt ? HXG_FP64_EXT_MIN_BLOCKS : HXG_FP64_MULTI_MIN_BLOCKS)
+shell_fp64_group_kernel(const __grid_constant__ PlanGroup<NF> G) {
+  unsigned block;
+  const int k = group_plan(G, block);
+  fp64_tile<NG, kExt, NF, kFast>(G.P[k], G.F[k],
+                                 ((long long)block * blockDim.x + threadIdx.x) >> 5,
+                                 threadIdx.x & 31);
+}
+
 }  // namespace hxg

@@ -172,6 +172,27 @@ __host__ __device__ __forceinline__ void freq_of_launch(const ShellLaunch &P, Fr
   Fq.out[0][2] = P.out[4];
 }
 
+// Shell launches of one instantiation in one kernel: plan k takes the blocks before
+// end[k] that the plans before it leave.  A kernel parameter, so that the plans'
+// values stay in constant memory.
+constexpr int kGroupPlans = 16;
+template <int NF>
+struct PlanGroup {
+  unsigned end[kGroupPlans];
+  ShellLaunch P[kGroupPlans];
+  FreqSet<NF> F[kGroupPlans];
+};
+static_assert(sizeof(PlanGroup<3>) <= 32764, "kernel parameters");
+
+// The plan of this block and the block's place in it.
+template <int NF>
+__device__ __forceinline__ int group_plan(const PlanGroup<NF> &G, unsigned &block) {
+  int k = 0;
+  while (k < kGroupPlans - 1 && blockIdx.x >= G.end[k]) ++k;
+  block = blockIdx.x - (k ? G.end[k - 1] : 0u);
+  return k;
+}
+
 // NESTED index of the shard's local pixel `local`: local pixels run through
 // the shard's blocks in order.
 __device__ __forceinline__ unsigned long long shard_nest(const ShellLaunch &P,

@@ -70,6 +70,14 @@ cudaError_t launch_shell64_multi(cudaStream_t s, const ShellLaunch &P, int nf, c
 // FreqSet<nf> (hxg_integrate.cuh).
 cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, int nf,
                                const void *fq, unsigned blocks, unsigned threads);
+// A number for the instantiation that a launch of P takes, and the plans of one
+// instantiation in one kernel: g points to a PlanGroup<nf>, P is one of its plans.
+int shell_instance(bool fp32, const ShellLaunch &P);
+int shell64_instance(const ShellLaunch &P);
+cudaError_t launch_shell_group(cudaStream_t s, bool fp32, int nf, const ShellLaunch &P,
+                               const void *g, unsigned blocks, unsigned threads);
+cudaError_t launch_group64(cudaStream_t s, int nf, const ShellLaunch &P, const void *g,
+                           unsigned blocks, unsigned threads);
 cudaError_t launch_accumulate_transpose(cudaStream_t s, int nside_out,
                                         int nside_shell, const double *g_out,
                                         double *g_shell, double scale);

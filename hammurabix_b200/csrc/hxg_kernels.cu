@@ -527,6 +527,29 @@ cudaError_t launch_shell_multi(cudaStream_t s, bool fp32, const ShellLaunch &P, 
   });
 }
 
+int shell_instance(bool fp32, const ShellLaunch &P) {
+  return fp32 ? shell_key(P.ngroups, P.ext != nullptr, fast_models(P) && P.fast_ok)
+              : shell64_instance(P);
+}
+
+cudaError_t launch_shell_group(cudaStream_t s, bool fp32, int nf, const ShellLaunch &P,
+                               const void *g, unsigned blocks, unsigned threads) {
+  if (!fp32) return launch_group64(s, nf, P, g, blocks, threads);
+  const bool fast = fast_models(P) && P.fast_ok;
+  return by_shape(P.ngroups, P.ext != nullptr, [&](auto ng, auto ext) {
+    constexpr int NG = decltype(ng)::value;
+    constexpr bool E = decltype(ext)::value;
+    by_passes(nf, [&](auto f) {
+      constexpr int NF = decltype(f)::value;
+      const auto &G = *static_cast<const PlanGroup<NF> *>(g);
+      if (fast)
+        shell_fp32c_group_kernel<NG, false, NF, true><<<blocks, threads, 0, s>>>(G);
+      else
+        shell_fp32c_group_kernel<NG, E, NF, false><<<blocks, threads, 0, s>>>(G);
+    });
+  });
+}
+
 cudaError_t launch_batch_level(cudaStream_t s, int ngroups, bool ext, bool fast,
                                const BatchLevel &B, unsigned blocks) {
   return by_shape(ngroups, ext, [&](auto ng, auto ex) {

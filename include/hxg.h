@@ -456,19 +456,19 @@ int hxg_adjoint_shard_finish(hxg_handle *h, double *d_grad_params, double *d_gra
  *  - outputs are the caller's device maps (RING), distinct per entry;
  *  - the plan holds per-entry shell temporaries and launch blocks and a
  *    graph with, per shell level, the shell kernels of the parameter sets
- *    side by side (hundreds of small FP32C sets share one persistent kernel
- *    instead, whose warps take pixel tiles from a work counter) and one
- *    kernel that merges the shell maps into the outputs; an entry's outer
- *    shells read the Faraday depth its inner shells accumulated, as in
- *    write_grid;
+ *    side by side (up to 16 small sets in one; hundreds of small FP32C sets
+ *    share one persistent kernel instead, whose warps take pixel tiles from a
+ *    work counter) and one kernel that merges the shell maps into the
+ *    outputs; an entry's outer shells read the Faraday depth its inner shells
+ *    accumulated, as in write_grid;
  *  - up to three consecutive entries with the same models and geometry and
  *    synchrotron output (one parameter set at several frequencies, as
  *    hxg_write_grid_multi takes them; no CRE grid) share one traversal per
  *    shell;
  *  - tune != 0: the launch shapes (lanes per pixel x tiles per fetch of the
- *    persistent kernel) are timed once in hxg_batch_create and the fastest is
- *    kept; the FP64 form takes more lanes where its plans would not fill the
- *    device;
+ *    persistent kernel) that differ for these entries are timed once in
+ *    hxg_batch_create and the fastest is kept; the FP64 form takes more lanes
+ *    where its plans would not fill the device;
  *  - hxg_batch_run launches the graph on the handle's stream and does not
  *    synchronise; the entries' host data are not read again;
  *  - grids uploaded to the handle after hxg_batch_create with the same
@@ -483,9 +483,10 @@ typedef struct hxg_batch hxg_batch;
 int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
                      int tune, hxg_batch **out);
 int hxg_batch_run(hxg_batch *b);
-/* Launch shape in use (lanes per pixel, tiles per fetch), the number of
- * shapes timed and the best graph time (ms; 0 without tuning), and the
- * LOS samples one run covers.                                             */
+/* Launch shape in use (lanes per pixel of the plan with the most samples,
+ * tiles per fetch of the persistent kernel, 0 where no plan is on it), the
+ * number of shapes timed and the best graph time (ms; 0 without tuning), and
+ * the LOS samples one run covers.                                          */
 int hxg_batch_info(const hxg_batch *b, int *lanes_per_pixel, int *grain,
                    int *tried, double *best_ms, int64_t *samples);
 int hxg_batch_destroy(hxg_batch *b);
