@@ -3103,6 +3103,15 @@ void batch_drop_graph(hxg_batch *b) {
 int batch_capture(hxg_batch *b) {
   hxg_handle *h = b->h;
   batch_drop_graph(b);
+  // resident blocks of the persistent kernels in use
+  for (int k = 0; k < 3 * b->levels; ++k) {
+    const int c = k % 3;
+    if (b->nplans[k] == 0 || b->level_blocks[c] != 0) continue;
+    int per_sm = 0;
+    HXG_CK(c == 0 ? hxg::batch_level_occupancy(b->ngroups, b->ext_any, b->fast, &per_sm)
+                  : hxg::batch_multi_occupancy(b->ngroups, b->ext_any, b->fast, c + 1, &per_sm));
+    b->level_blocks[c] = (unsigned)std::max(1, per_sm) * (unsigned)h->sm_count;
+  }
   cudaStream_t s = h->stream;
   HXG_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = hxg::launch_batch_zero(s, static_cast<const ZeroJob *>(b->zeros.p),
@@ -3308,14 +3317,6 @@ int hxg_batch_create(hxg_handle *h, int n, const hxg_batch_entry_t *entries,
     if ((st = build_launch(h, E.models, E.obs, 0, L, step)) != HXG_OK) return bail(st);
     L.ext = uses_ext(E.models) ? static_cast<const ExtModels *>(b->ext.p) : nullptr;
     b->fast = b->fast && hxg::fast_models(L) && L.fast_ok;
-  }
-  cudaError_t ce = cudaSuccess;
-  for (int nf = 1; nf <= 3 && b->fp32; ++nf) {
-    int per_sm = 0;
-    ce = nf == 1 ? hxg::batch_level_occupancy(b->ngroups, b->ext_any, b->fast, &per_sm)
-                 : hxg::batch_multi_occupancy(b->ngroups, b->ext_any, b->fast, nf, &per_sm);
-    if (ce != cudaSuccess) return bail(cuda_fail(h, ce, "occupancy"));
-    b->level_blocks[nf - 1] = (unsigned)std::max(1, per_sm) * (unsigned)h->sm_count;
   }
   // launch shapes: lanes per pixel x tiles per work fetch; those that come to the same
   // launches (a grain that no plan has, lanes that short rays do not take) once

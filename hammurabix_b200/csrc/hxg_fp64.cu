@@ -5,11 +5,6 @@
 
 namespace hxg {
 
-static int shape64(const ShellLaunch &P) {
-  const DevGridGroup &G = P.groups[0];
-  return fp64_groups(P.ngroups, G.rec, G.nx, G.ny, G.nz);
-}
-
 cudaError_t launch_shell64(cudaStream_t s, const ShellLaunch &P, unsigned blocks,
                            unsigned threads) {
   const bool fast = fast_models(P) && P.fast_ok;
@@ -39,27 +34,6 @@ cudaError_t launch_shell64_multi(cudaStream_t s, const ShellLaunch &P, int nf, c
       shell_fp64_multi_kernel<NG, E, 2, false><<<blocks, threads, 0, s>>>(P, F2);
     else
       shell_fp64_multi_kernel<NG, E, 3, false><<<blocks, threads, 0, s>>>(P, F3);
-  });
-}
-
-int shell64_instance(const ShellLaunch &P) {
-  return shell_key(shape64(P), P.ext != nullptr, fast_models(P) && P.fast_ok);
-}
-
-cudaError_t launch_group64(cudaStream_t s, int nf, const ShellLaunch &P, const void *g,
-                           unsigned blocks, unsigned threads) {
-  const bool fast = fast_models(P) && P.fast_ok;
-  return by_shape(shape64(P), P.ext != nullptr, [&](auto ng, auto ext) {
-    constexpr int NG = decltype(ng)::value;
-    constexpr bool E = decltype(ext)::value;
-    by_passes(nf, [&](auto f) {
-      constexpr int NF = decltype(f)::value;
-      const auto &G = *static_cast<const PlanGroup<NF> *>(g);
-      if (fast)
-        shell_fp64_group_kernel<NG, false, NF, true><<<blocks, threads, 0, s>>>(G);
-      else
-        shell_fp64_group_kernel<NG, E, NF, false><<<blocks, threads, 0, s>>>(G);
-    });
   });
 }
 

@@ -36,6 +36,7 @@
 // bound the loop, each about 60 % busy.
 #pragma once
 
+#include "hxg_dispatch.cuh"
 #include "hxg_integrate.cuh"
 
 // Launch shape of the FP64 shell kernels: threads per block and the resident
@@ -519,6 +520,12 @@ __global__ void __launch_bounds__(HXG_FP64_THREADS,
 shell_fp64_multi_kernel(const ShellLaunch P, const FreqSet<NF> Fq) {
   fp64_tile<NG, kExt, NF, kFast>(P, Fq, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                                  threadIdx.x & 31);
+}
+
+// The grid-group count of P's instantiation.
+inline int shape64(const ShellLaunch &P) {
+  const DevGridGroup &G = P.groups[0];
+  return fp64_groups(P.ngroups, G.rec, G.nx, G.ny, G.nz);
 }
 
 // The plans of a batch level, kGroupPlans to a kernel.
