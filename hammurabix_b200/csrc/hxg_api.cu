@@ -57,10 +57,10 @@ struct Group {
 
 // Bytes of output maps up to which a host-buffer call copies them in one piece, and
 // the calls of a handle that do so through a pageable block before a pinned one is
-// made: pinning takes 1-3 ms once, and a copy of 0.5 MB then 20 us instead of 53 (111
-// as five copies into the caller's arrays), so by then the handle's calls have saved
-// more than it costs.  First call of a new handle, one pass of Nside 32: 0.9-1.1 ms
-// with direct copies, 1.8-3.9 ms with pinning in it, 0.65 ms now.
+// made, which takes 1-3 ms.  One pass of Nside 32 (0.5 MB in five maps): 0.29 ms with
+// copies into the caller's arrays, 0.22 through the block, 0.165 through pinned memory,
+// so that by then the handle's calls have saved about what pinning costs; the first
+// call of a handle 0.7-3.3 ms, 0.6 and 1.8-3.9.
 constexpr size_t kLanding = 1u << 20;
 constexpr int kPinAfter = 16;
 
@@ -1476,7 +1476,9 @@ unsigned shard_block_log2(uint64_t npix, uint32_t nshards) {
 // Whether rays of a launch can leave the cuts within their first 0.4.  A lone
 // FP32C adjoint shell to 30 kpc, cut from 0.33 on, takes 13.9 ms with a chunk per
 // block against 16.7; one to 20 kpc, cut from 0.5 on, 4.05 against 3.8 ms, so
-// it keeps a pixel's chunks in one warp.
+// it keeps a pixel's chunks in one warp.  Lone FP32C forward shells (Nside 64-256, 1-3
+// passes): to 25 kpc, cut from 0.4 on, 0.93-13.2 ms against 1.57-19.8, to 40 kpc
+// 0.95-13.1 against 2.24-24.3.
 bool cut_early(const ShellLaunch &F) {
   double r2 = 0.;
   for (int k = 0; k < 3; ++k) r2 += F.obs[k] * F.obs[k];

@@ -30,7 +30,8 @@
 // 34.4 ms before these, 19.4 ms with the sample arithmetic, 14.4 ms with the
 // window cut into chunks and the coefficients as constant operands (30 of 32
 // lanes active against 20), 13.1 ms with quarter warps of neighbouring rays at
-// 128 x 5, 11.6 ms with 32-byte record loads.  A sample is 170 FP64
+// 128 x 5, 11.6 ms with 32-byte record loads, all pass by pass; 6.7 ms with the two
+// passes fused.  A sample is 170 FP64
 // instructions, 85 clocks of an SM's FP64 pipes, and about as many of its L1
 // data stage (8 records of 32 bytes for each of 32 lanes); the two together
 // bound the loop, each about 60 % busy.
@@ -41,8 +42,8 @@
 
 // Launch shape of the FP64 shell kernels: threads per block and the resident
 // blocks per SM their register allocation must allow.  128 x 5 (96 registers,
-// 20 warps, no spills with one grid) runs the case above in 11.6 ms against
-// 12.4 ms at 128 x 4 and 12.1 ms at 128 x 6 (80 registers, spills).
+// 20 warps, no spills with one grid) runs the case above pass by pass in 11.6 ms
+// against 12.4 ms at 128 x 4 and 12.1 ms at 128 x 6 (80 registers, spills).
 #ifndef HXG_FP64_THREADS
 #define HXG_FP64_THREADS 128
 #endif
@@ -50,13 +51,15 @@
 #define HXG_FP64_MIN_BLOCKS 5
 #endif
 // With the Jaffe / JF12 / YMW16 models 128 x 4 (128 registers): the masked JF12
-// pass of hxg_models_ext.cuh in 2.03 ms against 2.10 ms at 128 x 5.
+// pass of hxg_models_ext.cuh in 2.03 ms against 2.10 ms at 128 x 5; 1 to 3 passes over
+// Nside 32/64/128 with Jaffe, JF12, YMW16 and their combinations, with and without a
+// grid, within 3 % of 128 x 5 either way and 3-14 % faster than 128 x 3.
 #ifndef HXG_FP64_EXT_MIN_BLOCKS
 #define HXG_FP64_EXT_MIN_BLOCKS 4
 #endif
-// The fused kernels: three passes over Nside 128-1024 on 512^3 grids 91.7 ms
-// (205.3 ms pass by pass; 94.4 at 128 x 4, 95.4 at 128 x 6), two passes over
-// the case above 6.8 ms (7.2, 7.1).
+// The fused kernels: three passes over Nside 128-1024 on 512^3 grids 91.7 ms (94.4 at
+// 128 x 4, 95.4 at 128 x 6), two passes over the case above 6.8 ms (7.2, 7.1); 92.5 and
+// 6.7 ms now (211 and 11.8 pass by pass).
 #ifndef HXG_FP64_MULTI_MIN_BLOCKS
 #define HXG_FP64_MULTI_MIN_BLOCKS 5
 #endif

